@@ -5,6 +5,8 @@ by the CUDA path and the CPU oracle.  Exact decimal arithmetic at 60 digits:
   LOGC[i]   -log(INVC[i]) as an unevaluated sum hi + lo of two doubles
   EXP2[j]   2**(j/64), j = 0..63, as hi + lo
 
+and, for the CUDA path, the same values again in rows of one entry each.
+
 Run: python gen_ipow_tables.py > ipow_tables.h
 """
 from decimal import Decimal, getcontext
@@ -52,6 +54,17 @@ def main():
     emit("IPOW_LOGC_LO", llo)
     emit("IPOW_EXP2_HI", ehi)
     emit("IPOW_EXP2_LO", elo)
+    # the same values in rows, one or two 16-byte loads per row (CUDA only)
+    out.append("#ifdef __CUDACC__")
+    out.append("__device__ static const double4 IPOW_LOG_ROW[128] = {   // INVC, LOGC_HI, LOGC_LO, 0")
+    for k in range(128):
+        out.append("    {%s, %s, %s, 0.0}," % (hexf(invc[k]), hexf(lhi[k]), hexf(llo[k])))
+    out.append("};")
+    out.append("__device__ static const double2 IPOW_EXP2_ROW[64] = {   // EXP2_HI, EXP2_LO")
+    for k in range(64):
+        out.append("    {%s, %s}," % (hexf(ehi[k]), hexf(elo[k])))
+    out.append("};")
+    out.append("#endif")
     print("\n".join(out))
 
 

@@ -90,6 +90,7 @@ struct DevParams {
   double eps_sing, eps_sing4, hstep, one_by_h;
   double cfl, max_dt, reconstr_coeff, theta;
   int limiter[10];
+  int all_minmod, pad_;   // every limiter is 1
   int bcW_flag[8], bcE_flag[8], bcS_flag[8], bcN_flag[8];
   double bcW_val[8], bcE_val[8], bcS_val[8], bcN_val[8];
   int energy_flag, alpha_flag, rheology_flag, rheology_model;
@@ -129,6 +130,41 @@ IMEX_HD double fmax_f(double a, double b) {
   return (b > a) ? b : a;
 }
 IMEX_DIV_FN double ddiv(double a, double b) { return a / b; }
+
+// Several IEEE quotients by one divisor: one division and four
+// multiply-adds per quotient, instead of a division sequence each (about 9
+// FP64 and 8 other instructions).
+//   y = RN(1/b), yl ~ 1/b - y;  q = RN(a*y + a*yl) is within 0.51 ulp of a/b;
+//   r = a - b*q is then exact in one fused multiply-add, and RN(q + r*y) is
+//   RN(a/b) (Markstein's theorem: y correctly rounded, q faithful).
+// The theorem wants no overflow, underflow or inexact remainder: b in
+// [2^-300, 2^300] and a in [2^-600, 2^600] in magnitude, tested on the high words
+// read as floats (ordered like the doubles' magnitudes; NaN fails), or a = +-0,
+// for which the sign is that of a (b > 0).  Outside, `ok` is cleared and the caller
+// takes the plain divisions.
+struct Recip {
+  double b, y, yl;
+};
+IMEX_HD float hi_mag(double a) { return fabsf(__int_as_float(__double2hiint(a))); }
+IMEX_HD Recip recip_pos(double b, bool& ok) {
+  Recip R;
+  R.b = b;
+  R.y = 1.0 / b;
+  R.yl = fma(-b, R.y, 1.0) * R.y;
+  const float x = __int_as_float(__double2hiint(b));   // b < 0 and NaN fail
+  ok = ok & (x >= __int_as_float(0x2d300000)) & (x < __int_as_float(0x52b00000));
+  return R;
+}
+IMEX_HD double quot(const Recip& R, double a, bool& ok) {
+  const int ah = __double2hiint(a);
+  const float x = fabsf(__int_as_float(ah));
+  const bool zero = ((ah & 0x7fffffff) | __double2loint(a)) == 0;
+  ok = ok & ((x >= __int_as_float(0x1a700000) && x < __int_as_float(0x65700000)) || zero);
+  const double q = fma(a, R.y, a * R.yl);
+  const double r = fma(-R.b, q, a);
+  const double s = fma(r, R.y, q);
+  return __hiloint2double((__double2hiint(s) & 0x7fffffff) | (ah & 0x80000000), __double2loint(s));
+}
 
 // x**y for the non-integer exponents of the mass-exchange closures
 // (settling drag, hindered settling, entrainment, inlet ramps).  Both the CPU
@@ -688,22 +724,16 @@ IMEX_HD double minmod_uniform(double v1, double v2, double v3, double dz, double
 }
 
 // ------------------------------------------------------ source boundary
-template <int NS>
-IMEX_HD void eval_source_bdry(const DevParams& P, double time, double vx, double vy,
-                              double* sb) {
-  constexpr int NV = 4 + NS;
+// The inlet's time ramp, the same for every inlet cell of a step.
+struct InletRamp {
+  double tc, tc15, tc05;   // t_coeff and its powers 1.5 and 0.5
+  int over;                // past the end of the source
+};
+__device__ __noinline__ void inlet_ramp(const DevParams& P, double time, InletRamp& R) {
   const double* tp = P.time_param;
-  if (time >= tp[3]) {
-    sb[0] = 0.0;
-    sb[1] = 0.0;
-    sb[2] = 0.0;
-    sb[3] = P.T_source;
-#pragma unroll
-    for (int i = 0; i < NS; ++i) sb[4 + i] = 0.0;
-    sb[NV] = 0.0;
-    sb[NV + 1] = 0.0;
-    return;
-  }
+  R.tc = R.tc15 = R.tc05 = 0.0;
+  R.over = time >= tp[3];
+  if (R.over) return;
   double t_rem = fmod(time, tp[0]);
   double t_coeff = 0.0;
   const double pi_g = 3.141592653589793;
@@ -717,16 +747,35 @@ IMEX_HD void eval_source_bdry(const DevParams& P, double time, double vx, double
     else if (t_rem <= tp[1])
       t_coeff = 0.5 * (1.0 + cos(pi_g * ((t_rem - tp[1]) / tp[2] + 1.0)));
   }
-  double tc15 = ipow(t_coeff, 1.5), tc05 = ipow(t_coeff, 0.5);
-  sb[0] = t_coeff * P.h_source;
-  sb[1] = tc15 * P.h_source * P.vel_source * vx;
-  sb[2] = tc15 * P.h_source * P.vel_source * vy;
+  R.tc = t_coeff;
+  R.tc15 = ipow(t_coeff, 1.5);
+  R.tc05 = ipow(t_coeff, 0.5);
+}
+
+template <int NS>
+IMEX_HD void eval_source_bdry(const DevParams& P, const InletRamp& R, double vx, double vy,
+                              double* sb) {
+  constexpr int NV = 4 + NS;
+  if (R.over) {
+    sb[0] = 0.0;
+    sb[1] = 0.0;
+    sb[2] = 0.0;
+    sb[3] = P.T_source;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) sb[4 + i] = 0.0;
+    sb[NV] = 0.0;
+    sb[NV + 1] = 0.0;
+    return;
+  }
+  sb[0] = R.tc * P.h_source;
+  sb[1] = R.tc15 * P.h_source * P.vel_source * vx;
+  sb[2] = R.tc15 * P.h_source * P.vel_source * vy;
   sb[3] = P.T_source;
 #pragma unroll
   for (int i = 0; i < NS; ++i)
-    sb[4 + i] = P.alpha_flag ? P.alphas_source[i] : t_coeff * P.h_source * P.alphas_source[i];
-  sb[NV] = tc05 * P.vel_source * vx;
-  sb[NV + 1] = tc05 * P.vel_source * vy;
+    sb[4 + i] = P.alpha_flag ? P.alphas_source[i] : R.tc * P.h_source * P.alphas_source[i];
+  sb[NV] = R.tc05 * P.vel_source * vx;
+  sb[NV + 1] = R.tc05 * P.vel_source * vy;
 }
 
 // --------------------------------------------------- speeds and fluxes

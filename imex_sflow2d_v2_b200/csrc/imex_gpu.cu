@@ -716,7 +716,11 @@ int imex_gpu_create(const ImexParams* p, const ImexStatic* s, int device, ImexCt
   P.max_dt = p->max_dt;
   P.reconstr_coeff = p->reconstr_coeff;
   P.theta = p->theta;
-  for (int i = 0; i < P.nv + 2; ++i) P.limiter[i] = p->limiter[i];
+  P.all_minmod = 1;
+  for (int i = 0; i < P.nv + 2; ++i) {
+    P.limiter[i] = p->limiter[i];
+    if (P.limiter[i] != 1) P.all_minmod = 0;
+  }
   for (int i = 0; i < P.nv; ++i) {
     P.bcW_flag[i] = p->bcW[i].flag;
     P.bcE_flag[i] = p->bcE[i].flag;
@@ -2313,6 +2317,7 @@ __global__ void __launch_bounds__(FLUX_THREADS)
     if (threadIdx.x == 0) tile_min[tile] = P.max_dt;
     return;
   }
+  bool ring_cell = false;
   for (int e = threadIdx.x; e < SW * SH; e += blockDim.x) {
     int lx = e % SW, ly = e / SW;
     int j = j0 + lx - HALO, k = k0 + ly - HALO;
@@ -2338,10 +2343,13 @@ __global__ void __launch_bounds__(FLUX_THREADS)
 #pragma unroll
     for (int i = 0; i < NP; ++i) S.tile.qp[i][ly][lx] = qpv[i];
     S.tile.info[ly][lx] = inf;
+    ring_cell |= (inf & CI_SRC_MASK) == 2;
   }
+  if (__syncthreads_or(P.radial_source_flag && ring_cell) && threadIdx.x == 0)
+    inlet_ramp(P, time, S.ramp);
   __syncthreads();
   for (int e = threadIdx.x; e < NXI + NYI; e += blockDim.x) {
-    double H[NV], amax = 0.0, aN, aP;
+    double H[NV], amax = 0.0;
     if (e < NXI) {
       int jj = e % (TX + 1), kk = e / (TX + 1);
       int ja = j0 + jj - 1, ka = k0 + kk, ia_x = jj - 1 + HALO, ia_y = kk + HALO;
@@ -2352,8 +2360,7 @@ __global__ void __launch_bounds__(FLUX_THREADS)
       bool sb = b_in && (S.tile.info[ia_y][ia_x + 1] & 128);
       if (!(sa || sb)) continue;
       double gcf = P.slope_correction_flag ? gcsx[(size_t)ka * (nx + 1) + (ja + 1)] : 1.0;
-      interface_flux<NS>(P, S.tile, 1, ia_x, ia_y, ja, ka, a_in, b_in, gcf, false, time, ring, H,
-                         amax, aN, aP);
+      interface_flux<NS>(P, S.tile, 1, ia_x, ia_y, ja, ka, gcf, false, ring, S.ramp, H, amax);
       S.ax[kk][jj] = amax;
     } else {
       int e2 = e - NXI;
@@ -2366,8 +2373,7 @@ __global__ void __launch_bounds__(FLUX_THREADS)
       bool sb = b_in && (S.tile.info[ia_y + 1][ia_x] & 128);
       if (!(sa || sb)) continue;
       double gcf = P.slope_correction_flag ? gcsy[(size_t)(ka + 1) * nx + ja] : 1.0;
-      interface_flux<NS>(P, S.tile, 2, ia_x, ia_y, ja, ka, a_in, b_in, gcf, false, time, ring, H,
-                         amax, aN, aP);
+      interface_flux<NS>(P, S.tile, 2, ia_x, ia_y, ja, ka, gcf, false, ring, S.ramp, H, amax);
       S.ay[kk][jj] = amax;
     }
   }

@@ -249,34 +249,26 @@ struct Tile {
   uint8_t info[TS::SH][TS::SW];
 };
 
-// Face states of one cell in one direction: W/E (dir 1) or S/N (dir 2).
+IMEX_NOINL double limit_call(double v1, double v2, double v3, double z1, double z2, double z3,
+                             int lim, double theta) {
+  return limit(v1, v2, v3, z1, z2, z3, lim, theta);
+}
+
+// The face values of variable i of one cell in one direction, W/E (dir 1) or
+// S/N (dir 2), by all of the reference's rules.
 // `stage` selects the RK-stage arrays' view of never-solved inlet-interior
 // neighbours (all zero) instead of the module qp view (zero with T_ambient).
+// Few cells come here (border, inlet), but a block waits for them, so the
+// variables of a cell are separate tasks (special_faces below).
 template <int NS, class TS>
-IMEX_FLAT void cell_faces(const DevParams& P, const Tile<NS, TS>& T, int lx, int ly, int j, int k,
-                           int dir, bool stage, double time, const RingCell* ring,
-                           double* Fm, double* Fp) {
+IMEX_NOINL void special_face(const DevParams& P, const Tile<NS, TS>& T, int lx, int ly, int j, int k,
+                             int dir, bool stage, const RingCell* ring, const InletRamp& ramp,
+                             int var, double& Fm, double& Fp) {
   constexpr int NV = 4 + NS, NP = 6 + NS;
   const uint8_t inf = T.info[ly][lx];
   const int scell = inf & CI_SRC_MASK;
   const bool rad = P.radial_source_flag != 0;
   const bool sE = inf & CI_E, sW = inf & CI_W, sS = inf & CI_S, sN = inf & CI_N;
-  double sb[NP];
-#pragma unroll
-  for (int i = 0; i < NP; ++i) sb[i] = 0.0;
-  if (rad && scell == 2) {
-    const RingCell* rc = find_ring(ring, P.n_ring, (long long)k * P.nx + j);
-    if (rc) {
-      int w = sE ? 0 : (sW ? 1 : (sS ? 2 : 3));
-      eval_source_bdry<NS>(P, time, rc->vx[w], rc->vy[w], sb);
-    }
-  }
-  auto nb = [&](int v, int d) -> double {
-    int cx = (dir == 1) ? lx + d : lx;
-    int cy = (dir == 1) ? ly : ly + d;
-    if (stage && (T.info[cy][cx] & CI_SRC_MASK) == 1 && rad) return 0.0;
-    return T.qp[v][cy][cx];
-  };
   const int J = j + 1, K = k + 1;  // Fortran indices
   const int n = (dir == 1) ? P.nx : P.ny;
   const int I = (dir == 1) ? J : K;
@@ -294,6 +286,23 @@ IMEX_FLAT void cell_faces(const DevParams& P, const Tile<NS, TS>& T, int lx, int
   const bool ring_m = rad && scell == 2 && ((dir == 1) ? (!sE && sW) : (sS));
   const bool ring_p = rad && scell == 2 && ((dir == 1) ? sE : (!sS && sN));
   const bool border_src = (dir == 1) && scell == 2;
+  double sb[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) sb[i] = 0.0;
+  if (rad && scell == 2) {
+    const RingCell* rc = find_ring(ring, P.n_ring, (long long)k * P.nx + j);
+    if (rc) {
+      int w = sE ? 0 : (sW ? 1 : (sS ? 2 : 3));
+      eval_source_bdry<NS>(P, ramp, rc->vx[w], rc->vy[w], sb);
+    }
+  }
+  auto sbv = [&](int i) {
+    double r = sb[0];
+#pragma unroll
+    for (int m = 1; m < NP; ++m)
+      if (m == i) r = sb[m];
+    return r;
+  };
   // stencil abscissae after the n_vars loop
   double z1, z2 = comp(I), z3;
   if (I == 1) {
@@ -307,89 +316,106 @@ IMEX_FLAT void cell_faces(const DevParams& P, const Tile<NS, TS>& T, int lx, int
     z3 = ring_p ? stag(I + 1) : comp(I + 1);
   }
   const double rc_d = P.reconstr_coeff * dh;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    double v2 = nb(i, 0), slope;
-    if (I == 1) {
-      if (border_src) {
-        slope = limit(sb[i], v2, nb(i, 1), z1, z2, z3, P.limiter[i], P.theta);
-      } else if (flagm[i] == 0) {
-        slope = limit(valm[i], v2, nb(i, 1), z1, z2, z3, P.limiter[i], P.theta);
-      } else if (flagm[i] == 1) {
-        slope = valm[i];
+  const int ox = (dir == 1) ? 1 : 0, oy = 1 - ox;
+  const bool hide = stage && rad;
+  const bool hide_m = hide && (T.info[ly - oy][lx - ox] & CI_SRC_MASK) == 1;
+  const bool hide_c = hide && scell == 1;
+  const bool hide_p = hide && (T.info[ly + oy][lx + ox] & CI_SRC_MASK) == 1;
+  // u and v at a border face come from that face's h, hu and hv: those first
+  const bool from_q = var >= NV && (I == 1 || I == n);
+  double fh = 0.0, fq = 0.0;
+#pragma unroll 1
+  for (int t = from_q ? 0 : 2; t < 3; ++t) {
+    const int i = (t == 0) ? 0 : ((t == 1) ? 1 + var - NV : var);
+    const double v2 = hide_c ? 0.0 : T.qp[i][ly][lx];
+    double v1 = hide_m ? 0.0 : T.qp[i][ly - oy][lx - ox];
+    double v3 = hide_p ? 0.0 : T.qp[i][ly + oy][lx + ox];
+    double zz3 = z3, slope = 0.0, vf = 0.0;
+    bool given = false;
+    if (i < NV) {
+      if (I == 1) {
+        if (border_src) {
+          v1 = sbv(i);
+        } else if (flagm[i] == 0) {
+          v1 = valm[i];
+        } else {
+          slope = (flagm[i] == 1) ? valm[i] : (v3 - v2) * one_by_d;
+          given = true;
+        }
+      } else if (I == n) {
+        if (border_src) {
+          v3 = sbv(i);
+        } else if (flagp[i] == 0) {
+          v3 = valp[i];
+        } else {
+          slope = (flagp[i] == 1) ? valp[i] : (v2 - v1) * one_by_d;
+          given = true;
+        }
       } else {
-        slope = (nb(i, 1) - nb(i, 0)) * one_by_d;
-      }
-    } else if (I == n) {
-      if (border_src) {
-        slope = limit(nb(i, -1), v2, sb[i], z1, z2, z3, P.limiter[i], P.theta);
-      } else if (flagp[i] == 0) {
-        slope = limit(nb(i, -1), v2, valp[i], z1, z2, z3, P.limiter[i], P.theta);
-      } else if (flagp[i] == 1) {
-        slope = valp[i];
-      } else {
-        slope = (nb(i, 0) - nb(i, -1)) * one_by_d;
+        if (ring_m) v1 = sbv(i);
+        if (ring_p) v3 = sbv(i);
       }
     } else {
-      double v1 = ring_m ? sb[i] : nb(i, -1);
-      double v3 = ring_p ? sb[i] : nb(i, 1);
-      slope = limit(v1, v2, v3, z1, z2, z3, P.limiter[i], P.theta);
+      // u and v with the limiters of hu and hv
+      if (dir == 1 && i == NV + 1 && rad && scell == 2 && I > 1 && I < n && !sE && sN && !sS &&
+          K > 1 && K < P.ny)
+        zz3 = y_stag(P, K + 1);  // x_stencil(3)=y_stag(k+1), src/solver_2d.f90:3616
+      if (from_q) vf = (fh <= 0.0) ? 0.0 : fq / fh;
+      if (I == 1) {
+        v1 = vf;
+      } else if (I == n) {
+        v3 = vf;
+      } else {
+        if (ring_m) v1 = sbv(i);
+        if (ring_p) v3 = sbv(i);
+      }
     }
-    double dq = rc_d * slope;
+    if (!given) slope = limit_call(v1, v2, v3, z1, z2, zz3, P.limiter[i], P.theta);
+    const double dq = rc_d * slope;
     double fm = v2 - dq, fp = v2 + dq;
-    const int ivel = (dir == 1) ? 1 : 2;  // hu clamp in x, hv clamp in y
-    if (I == 1) {
-      if (border_src) fm = sb[i];
-      else if (flagm[i] == 0) fm = valm[i];
-      else if (i == ivel) fm = fmin_f(fm, 0.0);
-    }
-    if (I == n) {
-      if (border_src) fp = sb[i];
-      else if (flagp[i] == 0) fp = valp[i];
-      else if (i == ivel) fp = fmax_f(fp, 0.0);
-    }
-    Fm[i] = fm;
-    Fp[i] = fp;
-  }
-  // u and v with the limiters of hu and hv
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int i = NV + a;
-    double zz1 = z1, zz3 = z3;
-    if (dir == 1 && a == 1 && rad && scell == 2 && I > 1 && I < n && !sE && sN && !sS &&
-        K > 1 && K < P.ny)
-      zz3 = y_stag(P, K + 1);  // x_stencil(3)=y_stag(k+1), src/solver_2d.f90:3616
-    double v2 = nb(i, 0), v1, v3;
-    if (I == 1) {
-      v1 = (Fm[0] <= 0.0) ? 0.0 : Fm[1 + a] / Fm[0];
-      v3 = nb(i, 1);
-    } else if (I == n) {
-      v1 = nb(i, -1);
-      v3 = (Fp[0] <= 0.0) ? 0.0 : Fp[1 + a] / Fp[0];
+    if (i < NV) {
+      const int ivel = (dir == 1) ? 1 : 2;  // hu clamp in x, hv clamp in y
+      if (I == 1) {
+        if (border_src) fm = sbv(i);
+        else if (flagm[i] == 0) fm = valm[i];
+        else if (i == ivel) fm = fmin_f(fm, 0.0);
+      }
+      if (I == n) {
+        if (border_src) fp = sbv(i);
+        else if (flagp[i] == 0) fp = valp[i];
+        else if (i == ivel) fp = fmax_f(fp, 0.0);
+      }
     } else {
-      v1 = ring_m ? sb[i] : nb(i, -1);
-      v3 = ring_p ? sb[i] : nb(i, 1);
+      if (I == 1) fm = vf;
+      else if (I == n) fp = vf;
     }
-    double slope = limit(v1, v2, v3, zz1, z2, zz3, P.limiter[i], P.theta);
-    double dq = rc_d * slope;
-    Fm[i] = v2 - dq;
-    Fp[i] = v2 + dq;
-    if (I == 1) Fm[i] = v1;
-    else if (I == n) Fp[i] = v3;
+    fq = (I == 1) ? fm : fp;
+    if (t == 0) fh = fq;
+    Fm = fm;
+    Fp = fp;
   }
   if (I > 1 && I < n) {
-    if (ring_p) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) Fp[i] = sb[i];
-    } else if (ring_m) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) Fm[i] = sb[i];
-    }
+    if (ring_p) Fp = sbv(var);
+    else if (ring_m) Fm = sbv(var);
   }
 }
 
-// One interface: left/lower state from cell a, right/upper from cell b.
-// Writes the KT flux H (n_vars) and max(|a+|,|a-|) for the CFL.
+// All face values of one cell, one after the other: F[0..NP) the minus face,
+// F[NP..2NP) the plus one.
+template <int NS, class TS>
+IMEX_NOINL void cell_faces(const DevParams& P, const Tile<NS, TS>& T, int lx, int ly, int j, int k,
+                           int dir, bool stage, const RingCell* ring, const InletRamp& ramp,
+                           double* F) {
+  constexpr int NP = 6 + NS;
+#pragma unroll 1
+  for (int i = 0; i < NP; ++i) {
+    double fm, fp;
+    special_face<NS, TS>(P, T, lx, ly, j, k, dir, stage, ring, ramp, i, fm, fp);
+    F[i] = fm;
+    F[NP + i] = fp;
+  }
+}
+
 // Limited MUSCL increments of one direction, precomputed once per cell for
 // the cells whose faces need none of cell_faces' special rules: not on the
 // domain border in that direction, not an inlet cell, no inlet-interior
@@ -400,118 +426,183 @@ IMEX_FLAT void cell_faces(const DevParams& P, const Tile<NS, TS>& T, int lx, int
 template <int NS, class TS = Shape32x8>
 struct SlopeTile {
   double dq[6 + NS][TS::TY + 2][TS::TX + 2];
+  // 0: no faces kept; 1: increments in dq; FACES0 + s: both faces in slot s of
+  // the special faces (see special_faces)
   uint8_t ok[TS::TY + 2][TS::TX + 2];
 };
+constexpr int FACES0 = 2;
 
+// limit() for one variable on any spacing and limiter (the increments below
+// that their inlined form does not cover).
+IMEX_NOINL double slope_general(const DevParams& P, double v1, double v2, double v3, double dz,
+                                bool uniform, double z1, double z2, double z3, int lim) {
+  return (uniform && lim == 1) ? minmod_uniform(v1, v2, v3, dz, z1, z2, z3, P.theta)
+                               : limit(v1, v2, v3, z1, z2, z3, lim, P.theta);
+}
+
+// What bounds this is instruction issue: one division per cell and direction
+// (Recip) serves all variables.  Minmod on equal spacings with finite differences of
+// ordinary size is inlined per variable; the other limiters and unequal (rounded)
+// spacings take a rolled loop, one to three divisions per cell; infinities, NaN,
+// tiny and huge differences are a call.
 template <int NS, class TS>
 __device__ __forceinline__ void precompute_slopes(const DevParams& P, const Tile<NS, TS>& T,
                                                   SlopeTile<NS, TS>& D, int dir, int j0, int k0,
-                                                  const uint8_t* __restrict__ mask) {
-  constexpr int NP = 6 + NS, TX = TS::TX, TY = TS::TY;
-  const int nx = P.nx, ny = P.ny;
+                                                  int* n_special, uint16_t* special, int cap) {
+  constexpr int NP = 6 + NS, TX = TS::TX, TY = TS::TY, SW = TS::SW;
+  constexpr int QV = TS::SW * TS::SH, DV = (TY + 2) * (TX + 2);   // doubles per variable
   const bool rad = P.radial_source_flag != 0;
-  const int rw = (dir == 1) ? TX + 2 : TX, rh = (dir == 1) ? TY : TY + 2;
-  for (int e = threadIdx.x; e < rw * rh; e += blockDim.x) {
-    const int lx = (dir == 1) ? 1 + e % rw : HALO + e % rw;
-    const int ly = (dir == 1) ? HALO + e / rw : 1 + e / rw;
+  const int n = (dir == 1) ? P.nx : P.ny;
+  const int off = (dir == 1) ? 1 : SW;
+  const double rc_d = P.reconstr_coeff * ((dir == 1) ? P.dx2 : P.dy2);
+  const int count = (dir == 1) ? (TX + 2) * TY : TX * (TY + 2);
+  for (int e = threadIdx.x; e < count; e += blockDim.x) {
+    const int lx = (dir == 1) ? 1 + e % (TX + 2) : HALO + e % TX;
+    const int ly = (dir == 1) ? HALO + e / (TX + 2) : 1 + e / TX;
     const int j = j0 + lx - HALO, k = k0 + ly - HALO;
     uint8_t ok = 0;
-    const int I = (dir == 1) ? j + 1 : k + 1, n = (dir == 1) ? nx : ny;
-    if (j >= 0 && j < nx && k >= 0 && k < ny && I > 1 && I < n) {
-      const uint8_t inf = T.info[ly][lx];
-      const int dx_ = (dir == 1) ? 1 : 0, dy_ = (dir == 1) ? 0 : 1;
+    const int I = (dir == 1) ? j + 1 : k + 1;
+    const int di = (ly - 1) * (TX + 2) + lx - 1;
+    if (j >= 0 && j < P.nx && k >= 0 && k < P.ny && n > 1) {
+      const uint8_t* inf = &T.info[ly][lx];
+      const uint8_t i2 = inf[0], i1 = inf[-off], i3 = inf[off];
       // an active interface on either side: the cell or a neighbour is solved
-      const bool used = (inf & 128) || (T.info[ly - dy_][lx - dx_] & 128) ||
-                        (T.info[ly + dy_][lx + dx_] & 128);
-      const bool plain = !(rad && (inf & CI_SRC_MASK) != 0) &&
-                         !(rad && (T.info[ly - dy_][lx - dx_] & CI_SRC_MASK) == 1) &&
-                         !(rad && (T.info[ly + dy_][lx + dx_] & CI_SRC_MASK) == 1);
-      if (used && plain) {
-        const double dh = (dir == 1) ? P.dx2 : P.dy2;
-        const double rc_d = P.reconstr_coeff * dh;
+      const bool used = ((i1 | i2 | i3) & 128) != 0;
+      const bool inner_near = rad && ((i1 & CI_SRC_MASK) == 1 || (i3 & CI_SRC_MASK) == 1);
+      const bool plain = I > 1 && I < n && !(rad && (i2 & CI_SRC_MASK) != 0) && !inner_near;
+      if (used && !plain && !(rad && (i2 & CI_SRC_MASK) == 1)) {
+        // a slot for its faces, two (stage and timestep views) beside the inlet interior
+        const int need = inner_near ? 2 : 1;
+        const int s = atomicAdd(n_special, need);
+        if (s + need <= cap) {
+          special[s] = (uint16_t)(di << 1);
+          if (need == 2) special[s + 1] = (uint16_t)((di << 1) | 1);
+          ok = (uint8_t)(FACES0 + s);
+        } else {
+          for (int m = s; m < cap; ++m) special[m] = 0xffff;
+        }
+      } else if (used && plain) {
         const double z1 = (dir == 1) ? x_comp(P, I - 1) : y_comp(P, I - 1);
         const double z2 = (dir == 1) ? x_comp(P, I) : y_comp(P, I);
         const double z3 = (dir == 1) ? x_comp(P, I + 1) : y_comp(P, I + 1);
-        const double dz = z3 - z2;
-        const bool uniform = (dz == z2 - z1) && (z3 > z2) && (z2 > z1);
+        const double dz = z3 - z2, dz1 = z2 - z1;
+        const bool uniform = (dz == dz1) && (z3 > z2) && (z2 > z1);
+        bool gen = true;
+        const Recip R3 = recip_pos(dz, gen);
+        const bool fast = gen && dz >= 1e-10 && dz1 >= 1e-10;
+        const double* v = &T.qp[0][ly][lx];
+        double* dq = &D.dq[0][0][0] + di;
+        const float big = __int_as_float(0x65700000);
+        if (uniform && P.all_minmod) {
+#pragma unroll
+          for (int i = 0; i < NP; ++i) {
+            const double v1 = v[i * QV - off], v2 = v[i * QV], v3 = v[i * QV + off];
+            // 0 for differences of opposite sign or a zero one, else the smaller
+            // difference's slope (minmod_uniform)
+            const double d3 = v3 - v2, d1 = v2 - v1;
+            const bool zero = d3 == 0.0 || d1 == 0.0;
+            const bool opp = (__double2hiint(d3) ^ __double2hiint(d1)) < 0;
+            bool in = fast && hi_mag(d3) < big && hi_mag(d1) < big;
+            double lim = 0.0;
+            if (!(in && (zero || opp))) {
+              lim = quot(R3, (fabs(d1) < fabs(d3)) ? d1 : d3, in);
+              if (!in) lim = slope_general(P, v1, v2, v3, dz, true, z1, z2, z3, 1);
+            }
+            dq[i * DV] = rc_d * lim;
+          }
+        } else {
+          const Recip R1 = recip_pos(dz1, gen), R13 = recip_pos(z3 - z1, gen);
 #pragma unroll 1
-        for (int i = 0; i < NP; ++i) {
-          const double v1 = T.qp[i][ly - dy_][lx - dx_], v2 = T.qp[i][ly][lx],
-                       v3 = T.qp[i][ly + dy_][lx + dx_];
-          const double lim = (uniform && P.limiter[i] == 1)
-                                 ? minmod_uniform(v1, v2, v3, dz, z1, z2, z3, P.theta)
-                                 : limit(v1, v2, v3, z1, z2, z3, P.limiter[i], P.theta);
-          D.dq[i][ly - 1][lx - 1] = rc_d * lim;
+          for (int i = 0; i < NP; ++i) {
+            const double v1 = v[i * QV - off], v2 = v[i * QV], v3 = v[i * QV + off];
+            const int l = P.limiter[i];
+            const double d3 = v3 - v2, d1 = v2 - v1;
+            bool in = gen && l >= 1 && l <= 4 && hi_mag(d3) < big && hi_mag(d1) < big;
+            const double a = quot(R3, d3, in), b = quot(R1, d1, in);
+            double lim;
+            if (l == 1) {
+              lim = minmod(a, b);
+            } else if (l == 2) {
+              lim = maxmod(minmod(a, 2.0 * b), minmod(2.0 * a, b));
+            } else {
+              const double c = quot(R13, v3 - v1, in);
+              lim = minmod(c, ((l == 3) ? P.theta : 2.0) * minmod(a, b));
+            }
+            if (!in) lim = slope_general(P, v1, v2, v3, dz, uniform, z1, z2, z3, l);
+            dq[i * DV] = rc_d * lim;
+          }
         }
         ok = 1;
       }
     }
-    D.ok[ly - 1][lx - 1] = ok;
+    (&D.ok[0][0])[di] = ok;
   }
 }
 
+// Both face states of an interface by the reference's full rules: Q[0..NP) on
+// the side of cell a (left/lower), Q[NP..2NP) on b's.
 template <int NS, class TS>
-IMEX_FLAT void interface_flux(const DevParams& P, const Tile<NS, TS>& T, int dir, int la_x,
-                               int la_y, int ja, int ka, bool a_in, bool b_in, double gcf,
-                               bool stage, double time, const RingCell* ring, double* H,
-                               double& amax_flux, double& aneg_out, double& apos_out,
-                               const SlopeTile<NS, TS>* D = nullptr) {
-  constexpr int NV = 4 + NS, NP = 6 + NS;
-  const int lb_x = (dir == 1) ? la_x + 1 : la_x, lb_y = (dir == 1) ? la_y : la_y + 1;
-  const int jb = (dir == 1) ? ja + 1 : ja, kb = (dir == 1) ? ka : ka + 1;
-  double QL[NP], QR[NP], tmpm[NP], tmpp[NP];
+IMEX_NOINL void interface_states(const DevParams& P, const Tile<NS, TS>& T, int dir, int la_x,
+                                 int la_y, int ja, int ka, bool stage, const RingCell* ring,
+                                 const InletRamp& ramp, double* Q) {
+  constexpr int NP = 6 + NS;
+  const int ox = (dir == 1) ? 1 : 0, oy = 1 - ox;
+  const int lb_x = la_x + ox, lb_y = la_y + oy, jb = ja + ox, kb = ka + oy;
+  const int n = (dir == 1) ? P.nx : P.ny, ia0 = (dir == 1) ? ja : ka;
+  const bool a_in = ia0 >= 0, b_in = ia0 + 1 < n;
   const bool rad = P.radial_source_flag != 0;
   const uint8_t ia = a_in ? T.info[la_y][la_x] : 0, ib = b_in ? T.info[lb_y][lb_x] : 0;
   const bool a_int = rad && a_in && (ia & CI_SRC_MASK) == 1;
   const bool b_int = rad && b_in && (ib & CI_SRC_MASK) == 1;
-  const uint8_t flag_b_m = (dir == 1) ? CI_W : CI_S;  // b's inlet lies on its minus side
-  const uint8_t flag_a_p = (dir == 1) ? CI_E : CI_N;
-  // reconstruction of the sides that need it, through one call site
+  // reconstruction of the sides that need it
   const bool comp_a = a_in && (!b_in || !a_int);
   const bool comp_b = b_in && (!a_in || !b_int);
+  double F[2 * NP];
 #pragma unroll 1
   for (int side = 0; side < 2; ++side) {
     if (!(side == 0 ? comp_a : comp_b)) continue;
-    const int sx = side ? lb_x : la_x, sy = side ? lb_y : la_y;
-    if (D && stage && D->ok[sy - 1][sx - 1]) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        const double v2 = T.qp[i][sy][sx], dq = D->dq[i][sy - 1][sx - 1];
-        tmpm[i] = v2 - dq;
-        tmpp[i] = v2 + dq;
-      }
-    } else {
-      cell_faces<NS>(P, T, sx, sy, side ? jb : ja, side ? kb : ka, dir, stage, time, ring,
-                     tmpm, tmpp);
-    }
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      if (side == 0) QL[i] = tmpp[i];   // a's plus face
-      else QR[i] = tmpm[i];             // b's minus face
-    }
+    cell_faces<NS, TS>(P, T, side ? lb_x : la_x, side ? lb_y : la_y, side ? jb : ja,
+                       side ? kb : ka, dir, stage, ring, ramp, F);
+    // a's plus face, b's minus face
+#pragma unroll 1
+    for (int i = 0; i < NP; ++i) Q[side * NP + i] = F[side ? i : NP + i];
   }
+  // -1: keep; 0: zero; 1: the other side's state
+  int fix_a = -1, fix_b = -1;
   if (!a_in) {  // domain boundary on the minus side: both states from b's minus face
-#pragma unroll
-    for (int i = 0; i < NP; ++i) QL[i] = QR[i];
+    fix_a = 1;
   } else if (!b_in) {
-#pragma unroll
-    for (int i = 0; i < NP; ++i) QR[i] = QL[i];
+    fix_b = 1;
   } else {
-    const bool have_a = comp_a, have_b = comp_b;
-    if (a_int) {
-      // never solved: only the ring copy of src/solver_2d.f90:3768-3771 fills it
-      bool copy = have_b && (ib & flag_b_m) && (ib & CI_SRC_MASK) == 2 &&
-                  ((dir == 1) ? !(ib & CI_E) : true);
-      if (dir == 2) copy = have_b && (ib & CI_S) && (ib & CI_SRC_MASK) == 2;
+    // never solved: only the ring copy of src/solver_2d.f90:3768-3771 fills it
+    if (a_int)
+      fix_a = comp_b && (ib & CI_SRC_MASK) == 2 &&
+              ((dir == 1) ? (ib & CI_W) && !(ib & CI_E) : (ib & CI_S) != 0);
+    if (b_int)
+      fix_b = comp_a && (ia & CI_SRC_MASK) == 2 &&
+              ((dir == 1) ? (ia & CI_E) != 0 : (ia & CI_N) && !(ia & CI_S));
+  }
+#pragma unroll 1
+  for (int i = 0; i < NP; ++i) {
+    if (fix_a >= 0) Q[i] = fix_a ? Q[NP + i] : 0.0;
+    if (fix_b >= 0) Q[NP + i] = fix_b ? Q[i] : 0.0;
+  }
+}
+
+// One interface by the reference's own sequence: the KT flux H (n_vars) and
+// max(|a+|,|a-|) for the CFL.
+template <int NS, class TS>
+IMEX_FLAT void interface_flux(const DevParams& P, const Tile<NS, TS>& T, int dir, int la_x,
+                              int la_y, int ja, int ka, double gcf, bool stage,
+                              const RingCell* ring, const InletRamp& ramp, double* H,
+                              double& amax_flux) {
+  constexpr int NV = 4 + NS, NP = 6 + NS;
+  double Q[2 * NP], QL[NP], QR[NP];
+  interface_states<NS, TS>(P, T, dir, la_x, la_y, ja, ka, stage, ring, ramp, Q);
 #pragma unroll
-      for (int i = 0; i < NP; ++i) QL[i] = copy ? QR[i] : 0.0;
-    }
-    if (b_int) {
-      bool copy = have_a && (ia & flag_a_p) && (ia & CI_SRC_MASK) == 2;
-      if (dir == 2) copy = have_a && (ia & CI_N) && !(ia & CI_S) && (ia & CI_SRC_MASK) == 2;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) QR[i] = copy ? QL[i] : 0.0;
-    }
+  for (int i = 0; i < NP; ++i) {
+    QL[i] = Q[i];
+    QR[i] = Q[NP + i];
   }
   double cL[NV], cR[NV];
   Mixt mL, mR;
@@ -522,8 +613,6 @@ IMEX_FLAT void interface_flux(const DevParams& P, const Tile<NS, TS>& T, int dir
   local_speeds<NS>(P, QR, mR, gcf, dir, rmin, rmax);
   double aN = fmin_f(fmin_f(lmin, rmin), 0.0);
   double aP = fmax_f(fmax_f(lmax, rmax), 0.0);
-  aneg_out = aN;
-  apos_out = aP;
   amax_flux = fmax_f(aP, -aN);
   double fL[NV], fR[NV];
   eval_fluxes<NS>(P, cL, QL, mL, gcf, dir, fL);
@@ -582,16 +671,19 @@ struct FluxShared {
     // before the slopes are first written
     alignas(128) double stage[4 + NS][TS::SH][TS::SW];
   };
-  union {
-    double Hx[4 + NS][TS::TY][TS::TX + 1];
-    double Hy[4 + NS][TS::TY + 1][TS::TX];
-  } H;
-  union {
-    double ax[TS::TY][TS::TX + 1];
-    double ay[TS::TY + 1][TS::TX];
-  } A;
+  // by interface number: x faces (TX+1 per row), then, in their place, y faces
+  static constexpr int NI = TS::NXI > TS::NYI ? TS::NXI : TS::NYI;
+  double H[4 + NS][NI];
+  double A[NI];
   double dtmin[TS::THREADS / 32];
   unsigned long long tma_bar;   // mbarrier of the TMA box
+  InletRamp ramp;               // set in tiles that see an inlet ring cell
+  // cells whose faces special_faces computes: how many per direction, and
+  // which (slope index * 2 + timestep view)
+  static constexpr int FACES = ((4 + NS) * NI) / (2 * (6 + NS)) < 128
+                                   ? ((4 + NS) * NI) / (2 * (6 + NS)) : 128;
+  int n_special[2];
+  uint16_t special[FACES];
 };
 static_assert(Shape32x8::THREADS == 288, "k_flux blocks of 288 threads for 32x8 tiles");
 
@@ -621,7 +713,267 @@ struct CflShared {
   double ax[TY][TX + 1];
   double ay[TY + 1][TX];
   double dtmin[FLUX_THREADS / 32];
+  InletRamp ramp;
 };
+
+// One side of a plain interface: the conserved variables c of the face state
+// (normal and tangential momentum in cn, ct), its flux's velocity and pressure
+// term and its characteristic speeds.  The operations are those of
+// face_qc_mixt, local_speeds and eval_fluxes in both directions (in y the
+// normal momentum is hv and the celerity is sqrt((gcf*g')*h)); quotients by h
+// and by rho_m share a division (Recip).  A face that needs anything else (h not
+// above EPS by being NaN, a quotient out of Recip's range, solids above the
+// mixture's mass flux) clears ok.
+template <int NS>
+struct FaceSide {
+  double m, cn, ct, en, cs[NS];   // conserved variables
+  double vel, pres, lo, hi;       // flux velocity, pressure term, speeds
+};
+template <int NS>
+IMEX_FLAT void face_side(const DevParams& P, double h, double qn, double qt, double T,
+                         const double* qs, double un, double ut, double gcf, int dir,
+                         FaceSide<NS>& f, bool& ok) {
+  if (!(h > EPS)) {
+    ok = ok & (h <= EPS) & (0.0 * h * gcf == 0.0);   // NaN and infinite values
+    f.m = f.cn = f.ct = f.en = 0.0;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) f.cs[i] = 0.0;
+    // red_grav is 0: the celerity sqrt(0*h*gcf) is 0 (or takes the other branch)
+    f.vel = f.pres = 0.0;
+    f.lo = f.hi = un;
+    return;
+  }
+  double at = 0.0, al[NS];
+  if (P.alpha_flag) {
+#pragma unroll
+    for (int i = 0; i < NS; ++i) al[i] = qs[i];
+  } else if (NS == 1) {
+    al[0] = qs[0] / h;
+  } else {
+    const Recip Rh = recip_pos(h, ok);
+#pragma unroll
+    for (int i = 0; i < NS; ++i) al[i] = quot(Rh, qs[i], ok);
+  }
+#pragma unroll
+  for (int i = 0; i < NS; ++i) at += al[i];
+#pragma unroll
+  for (int i = 0; i < NS; ++i) al[i] = al[i] * P.rho_s[i];
+  const double rho_a = P.pres / (P.sp_gas_const_a * T);
+  const double rho_c = ((((1.0 - 0.0) - at) - 0.0) * rho_a + 0.0) / ((1.0 - 0.0) - at);
+  const double alc = 1.0 - at;
+  double sar = 0.0;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) sar += al[i];
+  const double rho_m = alc * rho_c + sar;
+  const Recip Rm = recip_pos(rho_m, ok);
+  const double rg = quot(Rm, rho_m - P.rho_a_amb, ok) * P.grav;
+  const double inv = Rm.y;
+  const double xc = alc * rho_c * inv;
+  const double cpc = (xc > EPS) ? ((xc - 0.0) * P.sp_heat_a + 0.0) / xc : P.sp_heat_a;
+  double dot = 0.0;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    al[i] = al[i] * inv;
+    dot += al[i] * P.sp_heat_s[i];
+  }
+  const double cpm = dot + xc * cpc;
+  f.m = rho_m * h;
+  f.cn = rho_m * qn;
+  f.ct = rho_m * qt;
+  f.en = P.energy_flag ? h * rho_m * (cpm * T + 0.5 * (un * un + ut * ut)) : h * rho_m * cpm * T;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) f.cs[i] = al[i] * f.m;
+  f.vel = un;
+  if (rg * h < 0.0) {
+    f.lo = f.hi = un;
+  } else {
+    const double c = sqrt((dir == 1) ? rg * h * gcf : gcf * rg * h);
+    f.lo = un - c;
+    f.hi = un + c;
+  }
+  f.pres = 0.5 * rho_m * gcf * rg * (h * h);
+  // the solids' flux cap (s/flux > 1, rounded, is s > flux for flux > 0)
+  const double f0 = un * f.m;
+  double fs = 0.0;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) fs += un * f.cs[i];
+  ok = ok & !(f0 > 0.0 && !(fs <= f0));
+}
+
+// A divergent solids' flux cap of the KT flux in S.H: s/H0 >= 1 in x, > 1 in y.
+template <int NS, class TS>
+IMEX_NOINL void cap_solids(FluxShared<NS, TS>& S, int dir, int e) {
+  const double H0 = S.H[0][e];
+  double s = 0.0, r = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < NS; ++i) s += S.H[4 + i][e];
+  const double q = s / H0;
+  if (!((dir == 1) ? q >= 1.0 : q > 1.0)) return;
+  if (dir == 1) {
+#pragma unroll 1
+    for (int i = 0; i < NS; ++i) r += S.H[4 + i][e] / H0;
+  } else {
+    r = q;
+  }
+#pragma unroll 1
+  for (int i = 0; i < NS; ++i) S.H[4 + i][e] = S.H[4 + i][e] / r;
+}
+
+// The faces of the tile's special cells (domain border, inlet ring and beside
+// the inlet), one thread per cell and variable, into the space of the
+// interface fluxes: slot s holds the minus face at 2*NP*s and the plus face NP
+// further.  One thread per interface used to do this for all variables of both
+// its cells in turn while the block waited: 42 of the 78 us that a corner
+// tile of a 200^2 grid took, 130 of 245 us beside an inlet.
+template <int NS, class TS>
+__device__ __forceinline__ void special_faces(const DevParams& P, FluxShared<NS, TS>& S, int n,
+                                              int dir, int j0, int k0,
+                                              const RingCell* __restrict__ ring) {
+  constexpr int NP = 6 + NS, W = TS::TX + 2;
+  double* F = &S.H[0][0];
+  for (int t = threadIdx.x; t < n * NP; t += blockDim.x) {
+    const int slot = t / NP, var = t - slot * NP;
+    const unsigned c = S.special[slot];
+    if (c == 0xffffu) continue;
+    const int di = c >> 1, lx = di % W + 1, ly = di / W + 1;
+    double fm, fp;
+    special_face<NS, TS>(P, S.tile, lx, ly, j0 + lx - HALO, k0 + ly - HALO, dir, (c & 1) == 0, ring,
+                         S.ramp, var, fm, fp);
+    F[slot * 2 * NP + var] = fm;
+    F[slot * 2 * NP + NP + var] = fp;
+  }
+}
+
+// Where an interface takes one side's face state from.
+enum FaceFrom { FACE_CELL, FACE_SLOT, FACE_OTHER, FACE_ZERO, FACE_NONE };
+
+// One side of an interface: the source of the face state of cell (x, y) of the
+// tile, `other` the cell across, in the stage or the timestep view.
+__device__ __forceinline__ FaceFrom face_from(bool rad, bool in, bool other_in, uint8_t inf,
+                                              uint8_t other_inf, uint8_t ok, int side, int dir) {
+  if (!in) return FACE_OTHER;            // domain boundary: both states from the inner cell
+  if (rad && (inf & CI_SRC_MASK) == 1) {
+    if (!other_in) return FACE_NONE;
+    // never solved: only the ring copy of src/solver_2d.f90:3768-3771 fills it
+    const bool ring = (other_inf & CI_SRC_MASK) == 2;
+    bool copy;
+    if (side == 0)   // a is inside: b's inlet lies on its minus side
+      copy = (dir == 1) ? (other_inf & CI_W) && !(other_inf & CI_E) : (other_inf & CI_S) != 0;
+    else
+      copy = (dir == 1) ? (other_inf & CI_E) != 0 : (other_inf & CI_N) && !(other_inf & CI_S);
+    return (ring && copy) ? FACE_OTHER : FACE_ZERO;
+  }
+  return ok == 1 ? FACE_CELL : (ok >= FACES0 ? FACE_SLOT : FACE_NONE);
+}
+
+// The KT flux of an interface (mass, normal and tangential momentum, energy,
+// solids) and its largest speed; false when the reference's own sequence is
+// needed (interface_special).  Plain interfaces take their faces from the cells'
+// values and increments (ia, ib: the cells in the tile, da, db: in the
+// slopes), the others as fromL/fromR say (slots sL, sR).
+// Before, four fifths of an interface's instructions were index arithmetic,
+// spills and the boundary and inlet rules inlined into it; now those rules
+// are separate tasks, the direction is an index, and the two sides' fluxes are
+// formed from c, the velocity and the pressure term when they are combined:
+// 1.04 against 2.01 ms for k_flux_tma<3> on 2048^2 cells.
+template <int NS, class TS>
+IMEX_FLAT bool interface_kt(const DevParams& P, const FluxShared<NS, TS>& S, int dir, FaceFrom fromL,
+                            FaceFrom fromR, int sL, int sR, int ia, int ib, int da, int db,
+                            double gcf, double* H, double& amax, bool& still) {
+  constexpr int NV = 4 + NS, NP = 6 + NS, QV = TS::SW * TS::SH, DV = (TS::TY + 2) * (TS::TX + 2);
+  const double* q = &S.tile.qp[0][0][0];
+  const double* d = &S.slopes.dq[0][0][0];
+  const double* F = &S.H[0][0];
+  const int vn = dir, vt = 3 - dir, wn = NV + dir - 1, wt = NV + 2 - dir;
+  bool ok = true;
+  FaceSide<NS> L, R;
+  double qnL, qnR;
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    // the cell, its increment or slot, and which face of it: its own side's, or
+    // (FACE_OTHER) the one the other side uses
+    const FaceFrom own = side ? fromR : fromL;
+    const bool swap = own == FACE_OTHER;
+    const FaceFrom from = swap ? (side ? fromL : fromR) : own;
+    const bool minus = (side == 1) != swap;
+    const int c = minus ? ib : ia, g = minus ? db : da, slot = minus ? sR : sL;
+    double h, qn, qt, T, un, ut, qs[NS];
+    if (from == FACE_CELL) {
+      auto face = [&](int v) {
+        const double a = q[v * QV + c], b = d[v * DV + g];
+        return minus ? a - b : a + b;
+      };
+      h = face(0);
+      qn = face(vn);
+      qt = face(vt);
+      T = face(3);
+#pragma unroll
+      for (int i = 0; i < NS; ++i) qs[i] = face(4 + i);
+      un = face(wn);
+      ut = face(wt);
+    } else {
+      const bool zero = from != FACE_SLOT;
+      const double* f = F + slot * 2 * NP + (minus ? 0 : NP);
+      auto face = [&](int v) { return zero ? 0.0 : f[v]; };
+      h = face(0);
+      qn = face(vn);
+      qt = face(vt);
+      T = face(3);
+#pragma unroll
+      for (int i = 0; i < NS; ++i) qs[i] = face(4 + i);
+      un = face(wn);
+      ut = face(wt);
+    }
+    (side ? qnR : qnL) = qn;
+    face_side<NS>(P, h, qn, qt, T, qs, un, ut, gcf, dir, side ? R : L, ok);
+  }
+  const double aN = fmin_f(fmin_f(L.lo, R.lo), 0.0);
+  const double aP = fmax_f(fmax_f(L.hi, R.hi), 0.0);
+  const double gap = aP - aN;
+  if (aN == aP) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) H[i] = 0.0;
+  } else {
+    const Recip Rg = recip_pos(gap, ok);
+    const double coef = quot(Rg, aP * aN, ok);
+    // products rounded on their own in the contracted build too: a multiply-add
+    // would round the two sides of the average differently, and the radial
+    // current amplifies that (relative L1 at step 500 2.2e-12 against 1.6e-12)
+    auto kt = [&](double fl, double fr, double cl, double cr) {
+      return quot(Rg, __dmul_rn(aP, fl) - __dmul_rn(aN, fr), ok) + __dmul_rn(coef, cr - cl);
+    };
+    H[0] = kt(L.vel * L.m, R.vel * R.m, L.m, R.m);
+    H[1] = kt(L.vel * L.cn + L.pres, R.vel * R.cn + R.pres, L.cn, R.cn);
+    H[2] = kt(L.vel * L.ct, R.vel * R.ct, L.ct, R.ct);
+    H[3] = P.energy_flag ? kt(L.vel * (L.en + L.pres), R.vel * (R.en + R.pres), L.en, R.en)
+                         : kt(L.vel * L.en, R.vel * R.en, L.en, R.en);
+#pragma unroll
+    for (int i = 0; i < NS; ++i) H[4 + i] = kt(L.vel * L.cs[i], R.vel * R.cs[i], L.cs[i], R.cs[i]);
+  }
+  amax = fmax_f(aP, -aN);
+  still = (dir == 1) ? (qnL == 0.0 && qnR == 0.0) : (L.cn == 0.0 && R.cn == 0.0);
+  return ok;
+}
+
+// An interface by the reference's own sequence (flux caps of a face state,
+// quotients outside Recip's range, NaN and infinite states).
+template <int NS, class TS>
+IMEX_NOINL void interface_special(const DevParams& P, FluxShared<NS, TS>& S, int dir, int e, int ax,
+                                  int ay, int ja, int ka, double gcf, bool again,
+                                  const RingCell* __restrict__ ring) {
+  constexpr int NV = 4 + NS;
+  double amax = 0.0;
+#pragma unroll 1
+  for (int pass = 0; pass < (again ? 2 : 1); ++pass) {
+    double H[NV];
+    interface_flux<NS, TS>(P, S.tile, dir, ax, ay, ja, ka, gcf, pass == 0, ring, S.ramp, H, amax);
+    if (pass == 0) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) S.H[i][e] = H[i];
+    }
+  }
+  S.A[e] = amax;
+}
 
 // Stage 1 and the CFL minimum on the tile whose first cell is (j0, k0).
 template <int NS, class TS>
@@ -676,7 +1028,9 @@ __device__ __forceinline__ void flux_tile(const DevParams& P, const double* __re
       return;
     }
   }
+  if (threadIdx.x == 0) S.n_special[0] = S.n_special[1] = 0;
   // physical states of the tile + halo
+  bool ring_cell = false;
   for (int e = threadIdx.x; e < SW * SH; e += blockDim.x) {
     int lx = e % SW, ly = e / SW;
     int j = j0 + lx - HALO, k = k0 + ly - HALO;
@@ -703,103 +1057,119 @@ __device__ __forceinline__ void flux_tile(const DevParams& P, const double* __re
 #pragma unroll
     for (int i = 0; i < NP; ++i) S.tile.qp[i][ly][lx] = qpv[i];
     S.tile.info[ly][lx] = inf;
+    ring_cell |= (inf & CI_SRC_MASK) == 2;
   }
-  __syncthreads();
-  // interfaces: x faces (e < NXI), then y faces, one interface per thread;
-  // each direction's slopes are precomputed once per cell first
-  const RingCell* rg = ring;
-  // this thread's cell (one per thread): the x part of the divergence and
+  // the inlet's time ramp once per block (used after the slopes' barrier)
+  if (__syncthreads_or(P.radial_source_flag && ring_cell) && threadIdx.x == 0)
+    inlet_ramp(P, time, S.ramp);
+  // interfaces: x faces, then y faces, one interface per thread; each
+  // direction's slopes are precomputed once per cell first.
+  // This thread's cell (one per thread): the x part of the divergence and
   // the x CFL dt, taken before the y phase reuses the flux arrays
   double dX[NV], dtx = P.max_dt;
-  for (int pdir = 1; pdir <= 2; ++pdir) {
-  precompute_slopes<NS>(P, S.tile, S.slopes, pdir, j0, k0, mask);
-  __syncthreads();
-  for (int e = (pdir == 1 ? 0 : NXI) + threadIdx.x; e < (pdir == 1 ? NXI : NXI + NYI);
-       e += blockDim.x) {
-    const int dir = (e < NXI) ? 1 : 2;
-    int jj, kk, ja, ka, ia_x, ia_y;
-    bool a_in, b_in, sa, sb_;
-    if (dir == 1) {
-      // interface between cells (j0+jj-1) and (j0+jj) in row k0+kk
-      jj = e % (TX + 1);
-      kk = e / (TX + 1);
-      ja = j0 + jj - 1;
-      ka = k0 + kk;
-      ia_x = jj - 1 + HALO;
-      ia_y = kk + HALO;
-    } else {
-      const int e2 = e - NXI;
-      jj = e2 % TX;
-      kk = e2 / TX;
-      ja = j0 + jj;
-      ka = k0 + kk - 1;
-      ia_x = jj + HALO;
-      ia_y = kk - 1 + HALO;
+#pragma unroll 1
+  for (int dir = 1; dir <= 2; ++dir) {
+    precompute_slopes<NS, TS>(P, S.tile, S.slopes, dir, j0, k0, &S.n_special[dir - 1], S.special,
+                              FluxShared<NS, TS>::FACES);
+    __syncthreads();
+    const int n_special = min(S.n_special[dir - 1], FluxShared<NS, TS>::FACES);
+    if (n_special) {
+      special_faces<NS, TS>(P, S, n_special, dir, j0, k0, ring);
+      __syncthreads();
     }
-    double& a_slot = (dir == 1) ? S.A.ax[kk][jj] : S.A.ay[kk][jj];
-    const bool exists = (dir == 1) ? !(ka >= ny || ja + 1 > nx) : !(ja >= nx || ka + 1 > ny);
+    const int count = (dir == 1) ? NXI : NYI, off = (dir == 1) ? 1 : SW,
+              doff = (dir == 1) ? 1 : TX + 2;
+    static_assert(NXI <= TS::THREADS && NYI <= TS::THREADS, "one interface per thread");
+    // this thread's interface.  x: between cells j0+jj-1 and j0+jj of row
+    // k0+kk; y: between rows k0+kk-1 and k0+kk of column j0+jj
+    const int e = threadIdx.x;
+    const int jj = (dir == 1) ? e % (TX + 1) : e % TX, kk = (dir == 1) ? e / (TX + 1) : e / TX;
+    const int ja = (dir == 1) ? j0 + jj - 1 : j0 + jj, ka = (dir == 1) ? k0 + kk : k0 + kk - 1;
+    const int ax = ja - j0 + HALO, ay = ka - k0 + HALO;
     // a direction of one cell has no fluxes and no speeds: the reference
     // skips its speeds, fluxes and divergence term (src/solver_2d.f90:
     // 2667-2681, 3946-4001), and its zero-initialised speed arrays give no
     // CFL limit there
-    const bool flat = (dir == 1) ? nx == 1 : ny == 1;
-    if (!exists || flat) { a_slot = 0.0; continue; }
-    if (dir == 1) {
-      a_in = ja >= 0;
-      b_in = ja + 1 < nx;
-      sa = a_in && (S.tile.info[ia_y][ia_x] & 128);
-      sb_ = b_in && (S.tile.info[ia_y][ia_x + 1] & 128);
-    } else {
-      a_in = ka >= 0;
-      b_in = ka + 1 < ny;
-      sa = a_in && (S.tile.info[ia_y][ia_x] & 128);
-      sb_ = b_in && (S.tile.info[ia_y + 1][ia_x] & 128);
-    }
-    if (!(sa || sb_)) { a_slot = 0.0; continue; }
-    double gcf = 1.0;
-    if (P.slope_correction_flag)
-      gcf = (dir == 1) ? gcsx[(size_t)ka * (nx + 1) + (ja + 1)] : gcsy[(size_t)(ka + 1) * nx + ja];
-    // CFL from the timestep view when an inlet-interior cell is in the stencil
-    bool dual = false;
-    if (P.radial_source_flag) {
-      for (int d = -1; d <= 2; ++d) {
-        const int cx = (dir == 1) ? ia_x + d : ia_x, cy = (dir == 1) ? ia_y : ia_y + d;
-        const int cg = (dir == 1) ? ja + d : ka + d, cn = (dir == 1) ? nx : ny;
-        if (cg >= 0 && cg < cn && (S.tile.info[cy][cx] & CI_SRC_MASK) == 1) dual = true;
+    const bool exists = e < count && ((dir == 1) ? !(ka >= ny || ja + 1 > nx || nx == 1)
+                                                 : !(ja >= nx || ka + 1 > ny || ny == 1));
+    // cells outside the grid have info 0
+    const uint8_t* inf = &S.tile.info[exists ? ay : 0][exists ? ax : 0];
+    const bool active = exists && ((inf[0] | inf[off]) & 128);
+    double H[NV], amax = 0.0, gcf = 1.0;
+    bool still = false, again = false, slow = false, slow2 = false;
+    if (active) {
+      if (P.slope_correction_flag)
+        gcf = (dir == 1) ? gcsx[(size_t)ka * (nx + 1) + (ja + 1)] : gcsy[(size_t)(ka + 1) * nx + ja];
+      const int ia = ay * SW + ax, da = (ay - 1) * (TX + 2) + ax - 1;
+      const uint8_t* sok = &S.slopes.ok[0][0];
+      const uint8_t oa = sok[da], ob = sok[da + doff];
+      FaceFrom fl = FACE_CELL, fr = FACE_CELL;
+      bool la = false, lb = false;   // the side's cell has a slot for the timestep view
+      if (!(oa == 1 && ob == 1)) {
+        const bool rad = P.radial_source_flag != 0;
+        const int n = (dir == 1) ? nx : ny, i0 = (dir == 1) ? ja : ka;
+        const bool a_in = i0 >= 0, b_in = i0 + 1 < n;
+        fl = face_from(rad, a_in, b_in, inf[0], inf[off], oa, 0, dir);
+        fr = face_from(rad, b_in, a_in, inf[off], inf[0], ob, 1, dir);
+        slow = fl == FACE_NONE || fr == FACE_NONE;
+        // the fluxes from the stage view; the CFL speeds from the timestep
+        // view (a second pass) when an inlet-interior cell is in the stencil
+        if (rad)
+          for (int m = -1; m <= 2; ++m)
+            if (i0 + m >= 0 && i0 + m < n && (inf[m * off] & CI_SRC_MASK) == 1) again = true;
+        la = again && a_in && i0 > 0 && (inf[-off] & CI_SRC_MASK) == 1;
+        la = la || (again && b_in && (inf[off] & CI_SRC_MASK) == 1);
+        lb = again && a_in && (inf[0] & CI_SRC_MASK) == 1;
+        lb = lb || (again && i0 + 2 < n && (inf[2 * off] & CI_SRC_MASK) == 1);
+      }
+      if (!slow) {
+        slow = !interface_kt<NS, TS>(P, S, dir, fl, fr, oa - FACES0, ob - FACES0, ia, ia + off, da,
+                                     da + doff, gcf, H, amax, still);
+        if (again) {
+          double H2[NV];
+          bool still2;
+          slow2 = !interface_kt<NS, TS>(P, S, dir, fl, fr, oa - FACES0 + la, ob - FACES0 + lb, ia,
+                                        ia + off, da, da + doff, gcf, H2, amax, still2);
+        }
       }
     }
-    double H[NV], amax = 0.0, aN, aP;
-#pragma unroll 1
-    for (int pass = 0; pass < (dual ? 2 : 1); ++pass) {
-      double Hp[NV];
-      interface_flux<NS>(P, S.tile, dir, ia_x, ia_y, ja, ka, a_in, b_in, gcf, pass == 0, time, rg,
-                         Hp, amax, aN, aP, &S.slopes);
-      if (pass == 0) {
+    // the special faces lie where the fluxes go
+    if (n_special) __syncthreads();
+    if (slow || slow2) {
+      interface_special<NS, TS>(P, S, dir, e, ax, ay, ja, ka, gcf, again, ring);
+    } else if (e < count) {
+      S.A[e] = amax;
+      if (active) {
+        const int vt = 3 - dir;
+        S.H[0][e] = H[0];
+        (&S.H[0][0])[dir * FluxShared<NS, TS>::NI + e] = H[1];
+        (&S.H[0][0])[vt * FluxShared<NS, TS>::NI + e] = H[2];
 #pragma unroll
-        for (int i = 0; i < NV; ++i) H[i] = Hp[i];
+        for (int i = 3; i < NV; ++i) S.H[i][e] = H[i];
+        // the cap on s/H0 needs |s| >= |H0| (rounded quotients are monotone)
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < NS; ++i) s += H[4 + i];
+        if (fabs(s) >= fabs(H[0]) && s != 0.0) cap_solids<NS, TS>(S, dir, e);
+        if (still) {
+          S.H[0][e] = 0.0;
+#pragma unroll
+          for (int i = 3; i < NV; ++i) S.H[i][e] = 0.0;
+        }
       }
     }
-    if (dir == 1) {
+    __syncthreads();
+    if (dir == 1 && threadIdx.x < TX * TY) {
+      const int e = threadIdx.x % TX + (threadIdx.x / TX) * (TX + 1);
 #pragma unroll
-      for (int i = 0; i < NV; ++i) S.H.Hx[i][kk][jj] = H[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) S.H.Hy[i][kk][jj] = H[i];
+      for (int i = 0; i < NV; ++i) {
+        double d = 0.0;
+        if (nx > 1) d = d + (S.H[i][e + 1] - S.H[i][e]) * P.one_by_dx;
+        dX[i] = d;
+      }
+      const double max_a = fmax_f(S.A[e], S.A[e + 1]);
+      dtx = (max_a > 0.0) ? P.cfl * P.dx / max_a : P.max_dt;
     }
-    a_slot = amax;
-  }
-  __syncthreads();
-  if (pdir == 1 && threadIdx.x < TX * TY) {
-    const int jj = threadIdx.x % TX, kk = threadIdx.x / TX;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      double d = 0.0;
-      if (nx > 1) d = d + (S.H.Hx[i][kk][jj + 1] - S.H.Hx[i][kk][jj]) * P.one_by_dx;
-      dX[i] = d;
-    }
-    const double max_a = fmax_f(S.A.ax[kk][jj], S.A.ax[kk][jj + 1]);
-    dtx = (max_a > 0.0) ? P.cfl * P.dx / max_a : P.max_dt;
-  }
   }
   // cells: divergence, explicit terms, CFL
   double dtl = P.max_dt;
@@ -828,10 +1198,10 @@ __device__ __forceinline__ void flux_tile(const DevParams& P, const double* __re
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       double d = dX[i];
-      if (ny > 1) d = d + (S.H.Hy[i][kk + 1][jj] - S.H.Hy[i][kk][jj]) * P.one_by_dy;
+      if (ny > 1) d = d + (S.H[i][e + TX] - S.H[i][e]) * P.one_by_dy;
       X[c + (size_t)i * P.plane] = d - ex[i];
     }
-    const double max_a = fmax_f(S.A.ay[kk][jj], S.A.ay[kk + 1][jj]);
+    const double max_a = fmax_f(S.A[e], S.A[e + TX]);
     double dty = (max_a > 0.0) ? P.cfl * P.dy / max_a : dtl;
     dtl = fmin_f(dtl, fmin_f(dtx, dty));
   }

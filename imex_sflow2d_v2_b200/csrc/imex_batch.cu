@@ -57,23 +57,21 @@ cudaError_t enqueue_ns(const Launch& L, int* launches) {
   kb_flux<NS, TS><<<wave(flux_min_blocks<NS, TS>()), TS::THREADS, smem, st>>>(
       M, L.tile_member, L.active, L.n_active);
   kb_dt_clip<<<mgrid, 128, 0, st>>>(M, n);
-  kb_stage2_first<NS><<<wave(IMEX_FIRST_MINB), STAGE2_THREADS, 0, st>>>(
-      M, L.tile_member, L.active, L.n_active, tx, ty);
-  for (int pass = 0; pass < 3; ++pass) {
-    kb_list_offsets<<<1, 1024, 0, st>>>(M, n, pass, L.list_off);
-    if (pass < 2)
-      kb_stage2_iter<NS><<<sms * IMEX_STAGE2_MINB, STAGE2_THREADS, 0, st>>>(M, n, L.list_off,
-                                                                              pass + 2);
-    else
-      kb_stage2_tail<NS><<<sms * IMEX_STAGE2_MINB, STAGE2_THREADS, 0, st>>>(M, n, L.list_off);
+  const int s2grid = wave(512 / STAGE2_THREADS);
+  kb_stage2<NS, false><<<s2grid, STAGE2_THREADS, 0, st>>>(M, L.tile_member, L.active, L.n_active,
+                                                          tx, ty);
+  *launches = 6 + (L.any_exchange ? 1 : 0);
+  if (tiles * tx * ty >= (long long)LIST_MIN_CELLS) {   // the step may use the list
+    kb_stage2<NS, true><<<s2grid, STAGE2_THREADS, 0, st>>>(M, L.tile_member, L.active, L.n_active,
+                                                           tx, ty);
+    kb_list_offsets<<<1, 1024, 0, st>>>(M, n, L.list_off);
+    kb_stage2_rest<NS><<<sms * IMEX_REST_MINB, STAGE2_THREADS, 0, st>>>(M, n, L.list_off);
+    *launches += 3;
   }
-  kb_stage2_post<NS><<<wave(8), STAGE2_THREADS, 0, st>>>(M, L.tile_member, L.active, L.n_active,
-                                                         tx, ty);
   if (L.any_exchange)
     kb_erosion<NS><<<wave(IMEX_EROSION_MINB), 128, 0, st>>>(M, L.tile_member, L.active,
                                                             L.n_active, tx, ty);
   kb_step_end<<<mgrid, 128, 0, st>>>(M, n);
-  *launches = 13 + (L.any_exchange ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -5,11 +5,11 @@
 // grid (a resident wave of blocks) walks a work list that the previous
 // phase built on the device.  The mask pass walks every tile of every member
 // and appends the tiles that hold a solve cell to the active-tile list; the
-// flux, stage-2 and erosion passes walk only those tiles; the Newton
-// iteration passes walk the members' Newton lists laid end to end.  The
-// per-tile and per-cell work is the single-grid path's own device code
-// (mask_tile, flux_tile, stage2_*_lane, stage2_post_cell,
-// erosion_update_cell), so a member advances bit for bit as it does alone.
+// flux, stage-2 and erosion passes walk only those tiles; the pass over the
+// cells that stage 2 left iterating walks the members' lists laid end to
+// end.  The per-tile and per-cell work is the single-grid path's own device code
+// (mask_tile, flux_tile, stage2_lane, stage2_rest_lane, erosion_update_cell),
+// so a member advances bit for bit as it does alone.
 //
 // The tile shape of the mask and flux passes is a template parameter: the
 // ensemble's tuner times a real step with each shape and keeps the fastest
@@ -150,51 +150,56 @@ __global__ void __launch_bounds__(TS::THREADS, (flux_min_blocks<NS, TS>()))
   }
 }
 
-// Stage 2 up to Newton iteration 1 on the cells of the active tiles (tiles
-// of tx x ty cells, walked in warp-sized runs of consecutive cells).
-template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_FIRST_MINB)
-    kb_stage2_first(const MemberDev* __restrict__ M, const uint32_t* __restrict__ tile_member,
-                    const uint32_t* __restrict__ active, const unsigned int* __restrict__ n_active,
-                    int tx, int ty) {
+// Stage 2 on the cells of the active tiles (tiles of tx x ty cells, walked in
+// warp-sized runs of consecutive cells).
+template <int NS, bool LIST>
+__global__ void __launch_bounds__(STAGE2_THREADS, 512 / STAGE2_THREADS)
+    kb_stage2(const MemberDev* __restrict__ M, const uint32_t* __restrict__ tile_member,
+              const uint32_t* __restrict__ active, const unsigned int* __restrict__ n_active,
+              int tx, int ty) {
   __shared__ DevParams sP;
+  __shared__ NewtonShared<NS, STAGE2_THREADS> S;
   const unsigned int n = *n_active;
+  // the active tiles' cells bound the members' solve cells together
+  if (((unsigned long long)n * (unsigned)(tx * ty) >= LIST_MIN_CELLS) != LIST) return;
   const MemberDev* cur = nullptr;
   for (unsigned int a = blockIdx.x; a < n; a += gridDim.x) {
     const TilePos t = tile_pos(M, tile_member, active[a], tx, ty);
     const MemberDev& D = *t.D;
     if (t.D != cur) {
       __syncthreads();
+      if (cur) stat_flush(S.st, cur->clk, threadIdx.x);
+      __syncthreads();
       stage_params(sP, D.P, threadIdx.x, blockDim.x);
+      stat_reset(S.st, threadIdx.x);
       __syncthreads();
       cur = t.D;
     }
     const double dt = D.clk->dt;
-    unsigned long long cells = 0, it_sum = 0, maxit = 0;
     for (int base = 0; base < tx * ty; base += blockDim.x) {
       const int e = base + threadIdx.x;
       const int j = t.j0 + e % tx, k = t.k0 + e / tx;
-      const bool valid = e < tx * ty && j < sP.nx && k < sP.ny;
-      const size_t c = valid ? (size_t)k * sP.pitch + j : 0;
-      stage2_first_lane<NS>(sP, D.q, D.X, D.mask, D.Bx, D.By, D.Bxx, D.Bxy, D.Byy, D.gc, D.W,
-                            D.clk, dt, valid, c, cells, it_sum, maxit);
+      stage2_lane<NS, STAGE2_THREADS, LIST>(sP, S, D.q, D.X, D.mask, D.cellinfo, D.Bx, D.By, D.Bxx,
+                                            D.Bxy, D.Byy, D.gc, D.W, D.clk, dt,
+                                            e < tx * ty && j < sP.nx && k < sP.ny, j, k);
     }
-    newton_flush_stats(D.clk, cells, it_sum, 0, maxit);
   }
+  __syncthreads();
+  if (cur) stat_flush(S.st, cur->clk, threadIdx.x);
 }
 
-// The members' lists `which` laid end to end, each padded to a multiple of
+// The members' lists laid end to end, each padded to a multiple of
 // 32 entries so that a warp never spans two members: off[m] is member m's
 // first slot, off[n] the total.  One block.
 __global__ void __launch_bounds__(1024)
-    kb_list_offsets(const MemberDev* __restrict__ M, int n, int which,
+    kb_list_offsets(const MemberDev* __restrict__ M, int n,
                     unsigned long long* __restrict__ off) {
   __shared__ unsigned long long warp_sum[32];
   const int per = (n + blockDim.x - 1) / blockDim.x;
   const int m0 = threadIdx.x * per;
   unsigned long long s = 0;
   for (int m = m0; m < m0 + per && m < n; ++m)
-    s += ((unsigned long long)M[m].clk->nw_count[which] + 31ULL) & ~31ULL;
+    s += ((unsigned long long)M[m].clk->nw_count[0] + 31ULL) & ~31ULL;
   // inclusive scan of s over the block
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned long long x = s;
@@ -216,7 +221,7 @@ __global__ void __launch_bounds__(1024)
   unsigned long long excl = x - s + (w > 0 ? warp_sum[w - 1] : 0ULL);
   for (int m = m0; m < m0 + per && m < n; ++m) {
     off[m] = excl;
-    excl += ((unsigned long long)M[m].clk->nw_count[which] + 31ULL) & ~31ULL;
+    excl += ((unsigned long long)M[m].clk->nw_count[0] + 31ULL) & ~31ULL;
   }
   if (threadIdx.x == blockDim.x - 1) off[n] = excl;
 }
@@ -232,13 +237,15 @@ __device__ __forceinline__ int list_member(const unsigned long long* __restrict_
   return lo;
 }
 
-// Newton iteration nl_iter (2 or 3) over the members' lists nl_iter-2.
+// The remaining Newton iterations and the assembly of the listed cells.
 template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
-    kb_stage2_iter(const MemberDev* __restrict__ M, int n, const unsigned long long* __restrict__ off,
-                   int nl_iter) {
+__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
+    kb_stage2_rest(const MemberDev* __restrict__ M, int n, const unsigned long long* __restrict__ off) {
   __shared__ DevParams sP[STAGE2_THREADS / 32];
+  __shared__ NewtonStats sst[STAGE2_THREADS / 32];   // a warp's, for its current member
+  const int lane = threadIdx.x & 31;
   DevParams& wP = sP[threadIdx.x >> 5];
+  NewtonStats& st = sst[threadIdx.x >> 5];
   int cur = -1;
   const unsigned long long total = off[n];
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -248,71 +255,19 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
     const MemberDev& D = M[m];
     if (m != cur) {
       __syncwarp();
-      stage_params(wP, D.P, threadIdx.x & 31, 32);
+      if (cur >= 0) stat_flush(st, M[cur].clk, lane);
+      __syncwarp();
+      stage_params(wP, D.P, lane, 32);
+      stat_reset(st, lane);
       __syncwarp();
       cur = m;
     }
-    const long long e = (long long)(base - off[m]) + (threadIdx.x & 31);
-    const bool valid = e < (long long)D.clk->nw_count[nl_iter - 2];
-    unsigned long long it_sum = 0, maxit = 0, trials = 0;
-    stage2_iter_lane<NS>(wP, D.q, D.Bx, D.By, D.W, D.clk, D.clk->dt, nl_iter, valid, e, it_sum,
-                         maxit, trials);
-    newton_flush_stats(D.clk, 0, it_sum, trials, maxit);
+    const long long e = (long long)(base - off[m]) + lane;
+    stage2_rest_lane<NS>(wP, D.q, D.cellinfo, D.Bx, D.By, D.W, D.clk, D.clk->dt,
+                         e < (long long)D.clk->nw_count[0], e, true, st);
   }
-}
-
-// Iterations 4..100 over the members' lists 2.
-template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
-    kb_stage2_tail(const MemberDev* __restrict__ M, int n, const unsigned long long* __restrict__ off) {
-  __shared__ DevParams sP[STAGE2_THREADS / 32];
-  DevParams& wP = sP[threadIdx.x >> 5];
-  int cur = -1;
-  const unsigned long long total = off[n];
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-       base < total; base += stride) {
-    const int m = list_member(off, n, base);
-    const MemberDev& D = M[m];
-    if (m != cur) {
-      __syncwarp();
-      stage_params(wP, D.P, threadIdx.x & 31, 32);
-      __syncwarp();
-      cur = m;
-    }
-    const long long e = (long long)(base - off[m]) + (threadIdx.x & 31);
-    const bool valid = e < (long long)D.clk->nw_count[2];
-    unsigned long long it_sum = 0, maxit = 0, trials = 0;
-    stage2_tail_lane<NS>(wP, D.q, D.Bx, D.By, D.W, D.clk, D.clk->dt, valid, e, it_sum, maxit,
-                         trials);
-    newton_flush_stats(D.clk, 0, it_sum, trials, maxit);
-  }
-}
-
-// Sign guard and assembly on the solve cells of the active tiles.
-template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS)
-    kb_stage2_post(const MemberDev* __restrict__ M, const uint32_t* __restrict__ tile_member,
-                   const uint32_t* __restrict__ active, const unsigned int* __restrict__ n_active,
-                   int tx, int ty) {
-  __shared__ DevParams sP;
-  const unsigned int n = *n_active;
-  const MemberDev* cur = nullptr;
-  for (unsigned int a = blockIdx.x; a < n; a += gridDim.x) {
-    const TilePos t = tile_pos(M, tile_member, active[a], tx, ty);
-    const MemberDev& D = *t.D;
-    if (t.D != cur) {
-      __syncthreads();
-      stage_params(sP, D.P, threadIdx.x, blockDim.x);
-      __syncthreads();
-      cur = t.D;
-    }
-    for (int e = threadIdx.x; e < tx * ty; e += blockDim.x) {
-      const int j = t.j0 + e % tx, k = t.k0 + e / tx;
-      if (j >= sP.nx || k >= sP.ny || !D.mask[(size_t)k * sP.pitch + j]) continue;
-      stage2_post_cell<NS>(sP, D.q, D.cellinfo, D.W, D.clk, j, k);
-    }
-  }
+  __syncwarp();
+  if (cur >= 0) stat_flush(st, M[cur].clk, lane);
 }
 
 // Erosion/deposition on the solve cells of the active tiles of the members

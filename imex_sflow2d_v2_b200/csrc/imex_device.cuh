@@ -101,6 +101,8 @@ struct DevParams {
   double rho_a_amb;
   double rho_s[MAXS], inv_rho_s[MAXS], diam_s[MAXS], sp_heat_s[MAXS];
   double mu, xi, friction_factor, maximum_solid_packing;
+  double xi_y, xi_yl;   // Recip of xi; xi_ok: in its range
+  int xi_ok, pad2_;
   double h_source, vel_source, T_source, alphas_source[MAXS], time_param[4];
   double erosion_coeff, erodible_porosity, T_erodible, alphastot_min;
   double erodible_fract[MAXS], rho_c_sub, coeff_porosity;
@@ -1060,6 +1062,248 @@ IMEX_RC_FN void implicit_terms_rc(const DevParams& P, double bx, double by, cons
   implicit_terms_c<NS>(P, bx, by, qc, pre, c2, c3);
   nh2 = c2.re;
   nh3 = c3.re;
+}
+
+// implicit_terms_r as a call, for the states the shorter forms below leave out.
+template <int NS>
+IMEX_NOINL void implicit_terms_any(const DevParams& P, double bx, double by, const double* q,
+                                   double* nh) {
+  implicit_terms_r<NS>(P, bx, by, q, nh[0], nh[1]);
+}
+
+IMEX_HD bool below_huge(double a) { return hi_mag(a) < __int_as_float(0x65700000); }  // 2^600
+
+// implicit_terms_r for ordinary states (q1 above eps_sing, every value finite
+// and of ordinary size), with quotients by one divisor sharing its division.
+// Same operations in the same order; false, and no result, for any other
+// state.  A value that is infinite or NaN leaves one of the tests below false: xc,
+// 1/rho and rho through Recip's range, the others by themselves or by what
+// is formed from them.
+template <int NS>
+IMEX_HD bool friction_real(const DevParams& P, double bx, double by, const double* q, double& nh2,
+                           double& nh3) {
+  nh2 = 0.0;
+  nh3 = 0.0;
+  if (!P.rheology_flag) return true;
+  bool ok = q[0] > P.eps_sing && q[0] > EPS;
+#pragma unroll
+  for (int i = 0; i < 4 + NS; ++i) ok = ok & below_huge(q[i]);
+  const double inv = 1.0 / q[0];
+  double xs_tot = 0.0, dot = 0.0, dot2 = 0.0;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    const double xs = q[4 + i] * inv;
+    xs_tot = xs_tot + xs;
+    dot = dot + xs * P.sp_heat_s[i];
+    dot2 = dot2 + xs * P.inv_rho_s[i];
+  }
+  const double xc = 1.0 - xs_tot;
+  const Recip Rx = recip_pos(xc, ok);
+  const double spc = quot(Rx, ((xc - 0.0) * P.sp_heat_a) + 0.0, ok);
+  const double sgc = quot(Rx, ((xc - 0.0) * P.sp_gas_const_a) + 0.0, ok);
+  const double spm = dot + xc * spc;
+  double Tn = q[3];
+  if (P.energy_flag) Tn = q[3] - ((q[1] * q[1] + q[2] * q[2]) * 0.5) * inv;
+  const double Td = q[0] * spm;
+  double T = Tn / Td;
+  ok = ok & below_huge(Td) & below_huge(T);
+  if (T <= 0.0) T = P.T_ambient;
+  const double irm = dot2 + xc * ((sgc * T) * P.inv_pres);
+  const double rho = 1.0 / irm;
+  const double u = q[1] * inv, v = q[2] * inv;
+  const Recip Rr = recip_pos(rho, ok);
+  const double rg = quot(Rr, rho - P.rho_a_amb, ok) * P.grav;
+  const double w = P.slope_correction_flag ? u * bx + v * by : 0.0;
+  const double mv2 = u * u + v * v + w * w;
+  ok = ok & below_huge(mv2);
+  if (mv2 != 0.0) {
+    if (P.rheology_model == 1) {
+      const Recip Rm = recip_pos(sqrt(mv2), ok), Rxi = {P.xi, P.xi_y, P.xi_yl};
+      const double ts = quot(Rxi, rho * rg, ok) * mv2;
+      ok = ok & below_huge(ts) & (P.xi_ok != 0);
+      nh2 = 0.0 - ts * quot(Rm, u, ok);
+      nh3 = 0.0 - ts * quot(Rm, v, ok);
+    } else if (P.rheology_model == 6) {
+      const Recip Rm = recip_pos(P.slope_correction_flag ? sqrt(u * u + v * v) : sqrt(mv2), ok);
+      nh2 = 0.0 - ((rho * quot(Rm, u, ok)) * P.friction_factor) * mv2;
+      nh3 = 0.0 - ((rho * quot(Rm, v, ok)) * P.friction_factor) * mv2;
+      ok = ok & below_huge(nh2) & below_huge(nh3);
+    }
+  }
+  return ok;
+}
+
+// friction_real together with the imaginary parts that implicit_terms_c gives for
+// the complex-step columns q2 + i*e2 and q3 + i*e3: nim[0], nim[1] are rows 2
+// and 3 of column 2, nim[2], nim[3] of column 3.
+// A perturbation is some 1e-15 of its component, so that in the products'
+// and Smith quotients' real parts the terms of second order round away, and all
+// real parts of both columns are those of the real evaluation.  Each such
+// equality is tested; with them, and with the parts that are zero by
+// construction left out, the remaining operations are those of implicit_terms_c.
+// The two columns and the real terms then share six divisions and one square root,
+// where the three evaluations made 54 and 5.
+// A momentum that has become small against its value at the solve's start
+// (a cell the friction stops) does perturb the speed's real part: with STOP
+// such a column takes its complex speed and the quotients by it in full, without
+// it false is returned.
+template <int NS, bool STOP = false>
+IMEX_HD bool friction_jacobian(const DevParams& P, double bx, double by, const double* q, double e2,
+                               double e3, double& nh2, double& nh3, double* nim) {
+  nh2 = 0.0;
+  nh3 = 0.0;
+  nim[0] = nim[1] = nim[2] = nim[3] = 0.0;
+  if (!P.rheology_flag) return true;
+  bool ok = q[0] > P.eps_sing && q[0] > EPS;
+#pragma unroll
+  for (int i = 0; i < 4 + NS; ++i) ok = ok & below_huge(q[i]);
+  // at rest the modulus' real part is 0 (the square root of -|e*inv|^2) and so
+  // is the friction
+  if (q[1] == 0.0 && q[2] == 0.0) return ok & below_huge(bx) & below_huge(by);
+  const double inv = 1.0 / q[0];
+  double xs_tot = 0.0, dot = 0.0, dot2 = 0.0;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    const double xs = q[4 + i] * inv;
+    xs_tot = xs_tot + xs;
+    dot = dot + xs * P.sp_heat_s[i];
+    dot2 = dot2 + xs * P.inv_rho_s[i];
+  }
+  const double xc = 1.0 - xs_tot;
+  const Recip Rx = recip_pos(xc, ok);
+  const double spc = quot(Rx, ((xc - 0.0) * P.sp_heat_a) + 0.0, ok);
+  const double sgc = quot(Rx, ((xc - 0.0) * P.sp_gas_const_a) + 0.0, ok);
+  const double spm = dot + xc * spc;
+  const double a2 = q[1] * q[1], b2 = q[2] * q[2], k2 = a2 + b2;
+  const Recip Rt = recip_pos(q[0] * spm, ok);
+  double T, Ti[2] = {0.0, 0.0};
+  if (P.energy_flag) {
+    T = quot(Rt, q[3] - (k2 * 0.5) * inv, ok);
+    const double im2 = q[1] * e2 + e2 * q[1], im3 = q[2] * e3 + e3 * q[2];
+    Ti[0] = quot(Rt, 0.0 - (im2 * 0.5) * inv, ok);
+    Ti[1] = quot(Rt, 0.0 - (im3 * 0.5) * inv, ok);
+  } else {
+    T = quot(Rt, q[3], ok);
+  }
+  ok = ok & (T > 0.0);
+  const double irm = dot2 + xc * ((sgc * T) * P.inv_pres);
+  const Recip Ri = recip_pos(irm, ok);
+  const double rho = Ri.y, dr = rho - P.rho_a_amb;
+  const Recip Rr = recip_pos(rho, ok);
+  const double rg = quot(Rr, dr, ok) * P.grav;
+  const double u = q[1] * inv, v = q[2] * inv;
+  const double w = P.slope_correction_flag ? u * bx + v * by : 0.0;
+  const double mv2 = u * u + v * v + w * w;
+  ok = ok & (mv2 > 0.0) & below_huge(mv2);
+  const double r = sqrt(mv2);
+  const Recip Rm = recip_pos(r, ok);
+  const double ur = quot(Rm, u, ok), vr = quot(Rm, v, ok);
+  const Recip Rxi = {P.xi, P.xi_y, P.xi_yl};
+  const bool voellmy = P.rheology_model == 1;
+  ok = ok & (!voellmy || P.xi_ok);
+  const double rr = rho * rg;
+  const double rrx = voellmy ? quot(Rxi, rr, ok) : 0.0;
+  const double ts = rrx * mv2;
+  // quadratic friction: the plane speed and what divides by it
+  const bool tilt = P.slope_correction_flag != 0;
+  const double p2 = u * u + v * v, rp = (!voellmy && tilt) ? sqrt(p2) : r;
+  Recip Rp = Rm;
+  double up = ur, vp = vr;
+  if (!voellmy && tilt) {
+    Rp = recip_pos(rp, ok);
+    up = quot(Rp, u, ok);
+    vp = quot(Rp, v, ok);
+  }
+  if (voellmy) {
+    nh2 = 0.0 - ts * ur;
+    nh3 = 0.0 - ts * vr;
+    ok = ok & below_huge(ts);
+  } else {
+    nh2 = 0.0 - ((rho * up) * P.friction_factor) * mv2;
+    nh3 = 0.0 - ((rho * vp) * P.friction_factor) * mv2;
+    ok = ok & below_huge(nh2) & below_huge(nh3);
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const double ui = (c == 0) ? e2 * inv : 0.0, vi = (c == 1) ? e3 * inv : 0.0;
+    // T's real part may differ, 1/rho's may not
+    const double kc = (c == 0) ? (a2 - e2 * e2) + b2 : a2 + (b2 - e3 * e3);
+    if (!STOP) {
+      ok = ok & (kc == k2);
+    } else if (P.energy_flag && kc != k2) {
+      const double Tc = quot(Rt, q[3] - (kc * 0.5) * inv, ok);
+      ok = ok & (Tc > 0.0) & (dot2 + xc * ((sgc * Tc) * P.inv_pres) == irm);
+    }
+    // rho = 1/irm
+    const double irmi = xc * ((sgc * Ti[c]) * P.inv_pres);
+    const double ra = quot(Ri, irmi, ok);
+    ok = ok & (irmi * ra + irm == irm);
+    const double rhoi = quot(Ri, 0.0 - ra, ok);
+    // red_grav = (rho - rho_a)/rho*grav
+    const double rb = quot(Rr, rhoi, ok);
+    const double t2 = rhoi * rb;
+    ok = ok & (t2 + rho == rho) & (t2 + dr == dr);
+    const double rgi = quot(Rr, rhoi - dr * rb, ok) * P.grav;
+    double rrxi = 0.0;
+    if (voellmy) {
+      const double rri = rho * rgi + rhoi * rg;
+      ok = ok & (rr - rhoi * rgi == rr);
+      rrxi = quot(Rxi, rri, ok);
+    }
+    // the speed and the quotients by it (xr, xi), (yr, yi)
+    const double wi = tilt ? ui * bx + vi * by : 0.0;
+    const double uu = u * u, vv = v * v, ww = w * w;
+    const double p2r = (uu - ui * ui) + (vv - vi * vi), m2r = p2r + (ww - wi * wi);
+    const double pi2 = (u * ui + ui * u) + (v * vi + vi * v);
+    const double m2i = pi2 + (w * wi + wi * w);
+    double xr = up, yr = vp, xi = 0.0, yi = 0.0;
+    bool small = (m2r == mv2) & (p2r == p2) & (mv2 * mv2 + m2i * m2i == mv2 * mv2) &
+                 (p2 * p2 + pi2 * pi2 == p2 * p2);
+    // sqrt(mv2*mv2) is mv2 itself there
+    small = small & (p2 > 1e-140) & (mv2 < 1e150);
+    {
+      const bool flat = voellmy || !tilt;
+      const double m = flat ? r : rp;
+      const Recip R = flat ? Rm : Rp;
+      const double mi = 0.5 * quot(R, flat ? m2i : pi2, small);
+      const double rc = quot(R, mi, small);
+      small = small & (mi * rc + m == m) & (ui * rc + u == u) & (vi * rc + v == v);
+      xi = quot(R, ui - u * rc, small);
+      yi = quot(R, vi - v * rc, small);
+    }
+    double tsr = ts, m2c = mv2;
+    if (!STOP) {
+      ok = ok & small;
+    } else if (!small) {
+      const cplx m2 = {m2r, m2i};
+      cplx s = csqrt_((voellmy || !tilt) ? m2 : cplx{p2r, pi2});
+      const cplx X = cplx{u, ui} / s, Y = cplx{v, vi} / s;
+      xr = X.re;
+      xi = X.im;
+      yr = Y.re;
+      yi = Y.im;
+      m2c = m2r;
+      tsr = rrx * m2r - rrxi * m2i;
+      // (a speed of real part 0 has no friction: left to the general call)
+      ok = ok & (s.re > 0.0) & below_huge(xr) & below_huge(xi) & below_huge(yr) & below_huge(yi);
+      if (!voellmy && tilt) ok = ok & (csqrt_(m2).re > 0.0);
+    }
+    if (voellmy) {
+      if (!STOP || small) ok = ok & (ts - rrxi * m2i == ts);
+      const double tsi = rrx * m2i + rrxi * m2c;
+      nim[2 * c] = 0.0 - (tsr * xi + tsi * xr);
+      nim[2 * c + 1] = 0.0 - (tsr * yi + tsi * yr);
+    } else {
+      // (rho*x)*ff*mv2
+      const double ax = rho * xr, ay = rho * yr;
+      ok = ok & (ax - rhoi * xi == ax) & (ay - rhoi * yi == ay);
+      const double axi = (rho * xi + rhoi * xr) * P.friction_factor;
+      const double ayi = (rho * yi + rhoi * yr) * P.friction_factor;
+      nim[2 * c] = 0.0 - ((ax * P.friction_factor) * m2i + axi * m2c);
+      nim[2 * c + 1] = 0.0 - ((ay * P.friction_factor) * m2i + ayi * m2c);
+    }
+  }
+  return ok;
 }
 
 template <int NS>

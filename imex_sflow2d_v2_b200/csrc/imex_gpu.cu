@@ -66,7 +66,7 @@ struct ImexCtx {
   uint32_t* post_vuln = nullptr;
   double* post_diag = nullptr;
   double* nw_buf = nullptr;      // backing store of nw's FP64 planes
-  uint32_t* nw_lists = nullptr;  // backing store of nw's three cell lists
+  uint32_t* nw_lists = nullptr;  // backing store of nw's cell list
   // learned warm start and training-pair harvest
   struct ImexMLP* warm_mlp = nullptr;  // not owned
   uint32_t* nw_wlist = nullptr;
@@ -159,9 +159,9 @@ int grid_1d(long long n, int threads) {
 enum {
   KID_MASK = 0,
   KID_FLUX = 1,
-  KID_S2_FIRST = 2,   // stage 2 up to Newton iteration 1
-  KID_S2_ITER = 3,    // Newton iterations 2.. (both list passes and the tail)
-  KID_S2_POST = 4,    // sign guard and assembly
+  KID_S2_FIRST = 2,   // stage 2 (with the learned start or harvest: up to iteration 1)
+  KID_S2_ITER = 3,    // the Newton iterations left to the list
+  KID_S2_POST = 4,    // sign guard and assembly (learned start, harvest)
   KID_EROSION = 5,
   KID_N = 6
 };
@@ -275,13 +275,60 @@ cudaError_t launch_flux(ImexCtx* ctx) {
 
 cudaError_t launch_warm_predict(ImexCtx* ctx);  // after ImexMLP (below)
 
+template <int NS, int T, bool LIST>
+cudaError_t launch_stage2_blocks(ImexCtx* ctx, int k0, int k1, unsigned long long list_min) {
+  const size_t smem = sizeof(NewtonShared<NS, T>);
+  static std::atomic<unsigned long long> attr{0};
+  if (attr_needed(attr)) {
+    cudaError_t e = cudaFuncSetAttribute(k_stage2<NS, T, LIST>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    attr_done(attr);
+  }
+  k_stage2<NS, T, LIST><<<grid_1d((long long)ctx->P.nx * (k1 - k0), T), T, smem, ctx->stream>>>(
+      ctx->P, ctx->q, ctx->X, ctx->mask, ctx->cellinfo, ctx->Bx, ctx->By, ctx->Bxx, ctx->Bxy,
+      ctx->Byy, ctx->gc, ctx->nw, ctx->clk, k0, k1, list_min);
+  ctx->launches += 1;
+  return cudaGetLastError();
+}
+
+// Stage 2 of the grid rows [k0, k1) (not with the learned start or harvest).  The
+// number of solve cells is known on the device only: a grid that can reach
+// LIST_MIN_CELLS gets both kernels, one of which returns at once (2 us).
+template <int NS>
+cudaError_t launch_stage2_rows(ImexCtx* ctx, int k0, int k1) {
+  const DevParams& P = ctx->P;
+  cudaError_t e;
+  if ((long long)P.nx * P.ny < (long long)LIST_MIN_CELLS) {
+    ProfScope ps(ctx, KID_S2_FIRST);
+    return launch_stage2_blocks<NS, STAGE2_THREADS, false>(ctx, k0, k1, ~0ULL);
+  }
+  k_nw_reset<<<1, 1, 0, ctx->stream>>>(ctx->clk);
+  ctx->launches += 1;
+  {
+    ProfScope ps(ctx, KID_S2_FIRST);
+    e = launch_stage2_blocks<NS, 512, true>(ctx, k0, k1, LIST_MIN_CELLS);
+    if (e == cudaSuccess)
+      e = launch_stage2_blocks<NS, STAGE2_THREADS, false>(ctx, k0, k1, LIST_MIN_CELLS);
+    if (e != cudaSuccess) return e;
+  }
+  ProfScope ps(ctx, KID_S2_ITER);
+  // one resident wave over the list
+  const int grid = grid_1d((long long)P.nx * (k1 - k0), STAGE2_THREADS);
+  k_stage2_rest<NS><<<std::min(grid, 148 * IMEX_REST_MINB), STAGE2_THREADS, 0, ctx->stream>>>(
+      ctx->P, ctx->q, ctx->cellinfo, ctx->Bx, ctx->By, ctx->nw, ctx->clk, 1);
+  ctx->launches += 1;
+  return cudaGetLastError();
+}
+
 template <int NS>
 cudaError_t launch_stage2_ns(ImexCtx* ctx) {
   const DevParams& P = ctx->P;
+  if (!ctx->nw.warm && !ctx->nw.harvest) return launch_stage2_rows<NS>(ctx, 0, P.ny);
   const long long ncell = (long long)P.nx * P.ny;
   const int grid = grid_1d(ncell, STAGE2_THREADS);
-  // list passes: one resident wave (IMEX_STAGE2_MINB blocks per SM), grid-stride
-  const int lgrid = std::min(grid, 148 * IMEX_STAGE2_MINB);
+  // list passes: one resident wave, grid-stride
+  const int lgrid = std::min(grid, 148 * IMEX_REST_MINB);
   k_nw_reset<<<1, 1, 0, ctx->stream>>>(ctx->clk);
   {
     ProfScope ps(ctx, KID_S2_FIRST);
@@ -298,12 +345,8 @@ cudaError_t launch_stage2_ns(ImexCtx* ctx) {
   }
   {
     ProfScope ps(ctx, KID_S2_ITER);
-    k_stage2_iter<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx,
-                                                                 ctx->By, ctx->nw, ctx->clk, 2);
-    k_stage2_iter<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx,
-                                                                 ctx->By, ctx->nw, ctx->clk, 3);
-    k_stage2_tail<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx,
-                                                                 ctx->By, ctx->nw, ctx->clk);
+    k_stage2_rest<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(
+        ctx->P, ctx->q, ctx->cellinfo, ctx->Bx, ctx->By, ctx->nw, ctx->clk, 0);
     if (ctx->nw.warm) {
       k_stage2_fallback<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx,
                                                                        ctx->By, ctx->nw, ctx->clk);
@@ -320,7 +363,7 @@ cudaError_t launch_stage2_ns(ImexCtx* ctx) {
     k_stage2_post<NS><<<grid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->mask,
                                                                 ctx->cellinfo, ctx->nw, ctx->clk);
   }
-  ctx->launches += 6;
+  ctx->launches += 4;
   return cudaGetLastError();
 }
 
@@ -454,9 +497,8 @@ constexpr int kHostBands = IMEX_HOST_BANDS;
 // run on the transfer stream; as band b has arrived and been converted,
 // the mask of band b-1 and the fluxes of band b-2 run (the mask needs two
 // rows of q beyond its band, the fluxes two rows of mask and q).  Stage 2
-// up to the Newton passes needs the global dt and runs on the whole grid;
-// then each band's assembly and erosion/deposition run and its rows go
-// back to the host while the next band computes.  Every cell sees the
+// needs the global dt; then each band's stage 2 and erosion/deposition run and
+// its rows go back to the host while the next band computes.  Every cell sees the
 // kernels and operations of enqueue_step, in the same order per cell.
 template <int NS>
 cudaError_t enqueue_host_step_ns(ImexCtx* ctx, const double* q_in, double* q_out) {
@@ -529,28 +571,10 @@ cudaError_t enqueue_host_step_ns(ImexCtx* ctx, const double* q_in, double* q_out
   flux_band(nb - 1);
   k_dt_clip<<<1, 1, 0, st>>>(ctx->clk, 1);
   ++launches;
-  // stage 2 through the Newton passes (launch_stage2_ns without assembly)
-  const long long ncell = (long long)P.nx * P.ny;
-  const int grid = grid_1d(ncell, STAGE2_THREADS);
-  const int lgrid = std::min(grid, 148 * IMEX_STAGE2_MINB);
-  k_nw_reset<<<1, 1, 0, st>>>(ctx->clk);
-  k_stage2_first<NS><<<grid, STAGE2_THREADS, 0, st>>>(ctx->P, ctx->q, ctx->X, ctx->mask, ctx->Bx,
-                                                     ctx->By, ctx->Bxx, ctx->Bxy, ctx->Byy,
-                                                     ctx->gc, ctx->nw, ctx->clk);
-  k_stage2_iter<NS><<<lgrid, STAGE2_THREADS, 0, st>>>(ctx->P, ctx->q, ctx->Bx, ctx->By, ctx->nw,
-                                                     ctx->clk, 2);
-  k_stage2_iter<NS><<<lgrid, STAGE2_THREADS, 0, st>>>(ctx->P, ctx->q, ctx->Bx, ctx->By, ctx->nw,
-                                                     ctx->clk, 3);
-  k_stage2_tail<NS><<<lgrid, STAGE2_THREADS, 0, st>>>(ctx->P, ctx->q, ctx->Bx, ctx->By, ctx->nw,
-                                                     ctx->clk);
-  launches += 5;
   const bool ero = erosion_active(ctx);
   for (int b = 0; b < nb; ++b) {
     const int k0 = r0(b), k1 = r1(b), rows = k1 - k0;
-    k_stage2_post_rows<NS><<<grid_1d((long long)rows * P.nx, STAGE2_THREADS), STAGE2_THREADS, 0,
-                             st>>>(ctx->P, ctx->q, ctx->mask, ctx->cellinfo, ctx->nw, ctx->clk, k0,
-                                   k1);
-    ++launches;
+    if ((e = launch_stage2_rows<NS>(ctx, k0, k1)) != cudaSuccess) return e;
     if (ero) {
       k_erosion_rows<NS><<<grid_1d((long long)rows * P.nx, 128), 128, 0, st>>>(
           ctx->P, ctx->q, ctx->mask, ctx->Bx, ctx->By, ctx->erodible, ctx->deposit, ctx->erosion,
@@ -760,6 +784,10 @@ int imex_gpu_create(const ImexParams* p, const ImexStatic* s, int device, ImexCt
   }
   P.mu = p->mu;
   P.xi = p->xi;
+  // Recip of xi (recip_pos)
+  P.xi_y = 1.0 / P.xi;
+  P.xi_yl = std::fma(-P.xi, P.xi_y, 1.0) * P.xi_y;
+  P.xi_ok = P.xi >= 0x1p-300 && P.xi < 0x1p300;
   P.friction_factor = p->friction_factor;
   P.maximum_solid_packing = p->maximum_solid_packing;
   P.h_source = p->h_source;
@@ -924,13 +952,13 @@ int imex_gpu_create(const ImexParams* p, const ImexStatic* s, int device, ImexCt
   // stage-2 Newton state: q_si, Rj, iterate, residual (nv planes each), |r|^2/2
   CK(dalloc(&ctx->nw_buf, plane * (4 * (size_t)nv + 1)));
   CK(dalloc(&ctx->nw.status, plane));
-  CK(dalloc(&ctx->nw_lists, plane * 3));
+  CK(dalloc(&ctx->nw_lists, plane));
   ctx->nw.qsi = ctx->nw_buf;
   ctx->nw.Rj = ctx->nw_buf + plane * nv;
   ctx->nw.x = ctx->nw_buf + plane * nv * 2;
   ctx->nw.rt = ctx->nw_buf + plane * nv * 3;
   ctx->nw.sf = ctx->nw_buf + plane * nv * 4;
-  for (int i = 0; i < 3; ++i) ctx->nw.list[i] = ctx->nw_lists + plane * i;
+  ctx->nw.list = ctx->nw_lists;
   CK(cudaDeviceSynchronize());
   *out = ctx;
   return IMEX_OK;

@@ -7,9 +7,8 @@
 //               boundary/inlet rules, local speeds, Kurganov-Tadmor fluxes,
 //               divergence, explicit terms and the CFL minimum
 //               (timestep + RK stage 1: src/solver_2d.f90:872-1005,2614-3918)
-//   k_stage2_*  RK stage 2: semi-implicit terms, Newton with line search and
-//               complex-step Jacobian (one pass per Newton iteration over the
-//               cells still iterating), assembly checks
+//   k_stage2    RK stage 2: semi-implicit terms, Newton with line search and
+//               complex-step Jacobian, assembly checks
 //               (src/solver_2d.f90:1105-1628, 1660-2365)
 //   k_erosion   the erosion/deposition update per cell
 //               (src/solver_2d.f90:2380-2595)
@@ -55,13 +54,8 @@ constexpr int FLUX_THREADS = Shape32x8::THREADS;
 constexpr int NXI = Shape32x8::NXI;
 constexpr int NYI = Shape32x8::NYI;
 
-// Minimum resident blocks per SM asked of ptxas for the flux and per-cell
-// kernels (their register budget); tuning knobs, set with -D at build time.
-// The Newton list passes run at 128 registers (4 blocks of 128): 7.34 ms
-// per step at 4096^2 against 7.63 at 96 registers and 7.79 at 80.
-#ifndef IMEX_STAGE2_MINB
-#define IMEX_STAGE2_MINB 4
-#endif
+// Minimum resident blocks per SM asked of ptxas for the per-cell kernels
+// (their register budget); tuning knobs, set with -D at build time.
 #ifndef IMEX_EROSION_MINB
 #define IMEX_EROSION_MINB 8
 #endif
@@ -494,7 +488,7 @@ __device__ __forceinline__ void precompute_slopes(const DevParams& P, const Tile
         double* dq = &D.dq[0][0][0] + di;
         const float big = __int_as_float(0x65700000);
         if (uniform && P.all_minmod) {
-#pragma unroll
+#pragma unroll 3
           for (int i = 0; i < NP; ++i) {
             const double v1 = v[i * QV - off], v2 = v[i * QV], v3 = v[i * QV + off];
             // 0 for differences of opposite sign or a zero one, else the smaller
@@ -1290,42 +1284,59 @@ __global__ void __launch_bounds__(FLUX_THREADS, flux_min_blocks<NS>())
 
 // =============================================================== Newton
 // solve_rk_step (src/solver_2d.f90:1660-1994) for a_diag = 1 (stage 2 of the
-// n_RK = 2 tableau), cut at its iteration boundaries: newton_start (scaling
-// and the test before the first iteration), newton_iter1 (the first
-// iteration, a full step) and newton_iterk (every later iteration, with the
-// line search).  The stage-2 passes below run one iteration per pass over a
-// compacted list of the cells still iterating; each cell goes through
-// exactly the operation sequence of one uninterrupted solve_rk_step.
+// n_RK = 2 tableau): newton_begin (scaling and start), then newton_step per
+// iteration.
 constexpr int NEWTON_MAX_IT = 100;
 constexpr double NEWTON_TOLF = 1.0e-10, NEWTON_STPMX = 100.0;
 
 #ifndef IMEX_EVAL_FN
 #define IMEX_EVAL_FN IMEX_FLAT
 #endif
-template <int NS>
-IMEX_EVAL_FN void eval_f(const DevParams& P, const double* qj, const double* qj_old,
-                       const double* Rj, double bx, double by, double dt, double* f,
-                       double& scal_f) {
+// Per-cell vectors that are only read during the solve (the old state, Rj, the
+// scaling) have a stride ST: 1 in registers, or the block size in shared memory
+// (NewtonShared).
+// The residual of qj with its implicit terms, and half its squared norm.
+template <int NS, int ST>
+IMEX_EVAL_FN void newton_residual(const double* qj, const double* qj_old, const double* Rj,
+                                  double nh2, double nh3, double dt, double* f, double& scal_f) {
   constexpr int NV = 4 + NS;
-  double nh2, nh3;
-  implicit_terms_r<NS>(P, bx, by, qj, nh2, nh3);
+  double d = 0.0;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     double nh = (i == 1) ? nh2 : ((i == 2) ? nh3 : 0.0);
-    double R = Rj[i] - 1.0 * nh;
-    double fi = qj[i] - qj_old[i] + dt * R;
-    f[i] = 1.0 * fi;
+    double R = Rj[i * ST] - 1.0 * nh;
+    double fi = qj[i] - qj_old[i * ST] + dt * R;
+    const double fs = 1.0 * fi;
+    f[i] = fs;
+    d += fs * fs;
   }
-  double d = 0.0;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) d += f[i] * f[i];
   scal_f = 0.5 * d;
+}
+// The implicit terms of a state outside friction_real's and
+// friction_jacobian's range.
+template <int NS>
+IMEX_FLAT void friction_any(const DevParams& P, double bx, double by, const double* qj, double& nh2,
+                            double& nh3) {
+  double t[4 + NS], nh[2];
+#pragma unroll
+  for (int i = 0; i < 4 + NS; ++i) t[i] = qj[i];
+  implicit_terms_any<NS>(P, bx, by, t, nh);
+  nh2 = nh[0];
+  nh3 = nh[1];
+}
+template <int NS, int ST>
+IMEX_EVAL_FN void eval_f(const DevParams& P, const double* qj, const double* qj_old,
+                       const double* Rj, double bx, double by, double dt, double* f,
+                       double& scal_f) {
+  double nh2, nh3;
+  if (!friction_real<NS>(P, bx, by, qj, nh2, nh3)) friction_any<NS>(P, bx, by, qj, nh2, nh3);
+  newton_residual<NS, ST>(qj, qj_old, Rj, nh2, nh3, dt, f, scal_f);
 }
 
 // Jacobian columns 2,3 by complex step (src/solver_2d.f90:2300-2365) and the
 // Newton direction: explicit rows diagonal, 2x2 Cramer on rows/cols 2,3
 // (src/solver_2d.f90:1879-1901).
-template <int NS, bool COLS_TOGETHER = false>
+template <int NS>
 IMEX_FLAT void newton_direction(const DevParams& P, double bx, double by, double dt,
                                               const double* qj_org, const double* qj_rel,
                                               const double* rt, double* dd, double* J2,
@@ -1354,15 +1365,8 @@ IMEX_FLAT void newton_direction(const DevParams& P, double bx, double by, double
       else J3[r] = v;
     }
   };
-  // the two columns one after the other, or (COLS_TOGETHER) unrolled, so
-  // that the scheduler may interleave their independent chains
-  if constexpr (COLS_TOGETHER) {
-#pragma unroll
-    for (int col = 1; col <= 2; ++col) column(col);
-  } else {
 #pragma unroll 1
-    for (int col = 1; col <= 2; ++col) column(col);
-  }
+  for (int col = 1; col <= 2; ++col) column(col);
   double d1[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) d1[i] = (i == 1 || i == 2) ? 0.0 : rt[i] / (1.0 * qj_org[i]);
@@ -1390,128 +1394,14 @@ IMEX_FLAT void newton_direction(const DevParams& P, double bx, double by, double
   }
 }
 
-// The exit tests at the end of an iteration (src/solver_2d.f90:1964-1988).
+// The direction and the gradient J^T rt by the general expressions, as a call:
+// in holds qj_org, qj_rel and rt, out receives dd and grad.
 template <int NS>
-__device__ __forceinline__ bool newton_converged(const double* rt, const double* qj_rel,
-                                                 const double* x_old) {
+IMEX_NOINL void newton_direction_any(const DevParams& P, double bx, double by, double dt,
+                                     const double* in, double* out) {
   constexpr int NV = 4 + NS;
-  double mx = fabs(rt[0]);
-#pragma unroll
-  for (int i = 1; i < NV; ++i) mx = fmax_f(mx, fabs(rt[i]));
-  if (mx < NEWTON_TOLF) return true;
-  // m3 = MAX over i of |qj_rel - x_old| / MAX(|qj_rel|, 1) < EPS.  MAX skips
-  // NaN quotients (all NaN: NaN, and the test fails), so the test holds when
-  // some quotient is a number and every such quotient is below EPS; each
-  // comparison of a rounded quotient is taken without the division where
-  // its answer is certain (rel_change_below).
-  bool any = false, below = true;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const double d = fabs(qj_rel[i] - x_old[i]), s = fmax_f(fabs(qj_rel[i]), 1.0);
-    if (isnan(d) || (isinf(d) && isinf(s))) continue;   // the quotient is NaN
-    any = true;
-    below = below & rel_change_below(d, s, EPS);
-  }
-  return any && below;
-}
-
-// Scaling (src/solver_2d.f90:1786-1798); the residual test before the first
-// Jacobian.  True: q already satisfies TOLF (exit with nl_iter = 1).
-template <int NS>
-__device__ __forceinline__ void newton_scale(const double* qj, double* qj_org) {
-  constexpr int NV = 4 + NS;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) qj_org[i] = fmax_f(fabs(qj[i]), 1.0e-3);
-}
-
-template <int NS>
-__device__ bool newton_start(const DevParams& P, const double* qj, const double* qj_old,
-                             const double* Rj, double bx, double by, double dt,
-                             const double* qj_org, double* qj_rel, double* rt, double& scal_f) {
-  constexpr int NV = 4 + NS;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) qj_rel[i] = qj[i] / qj_org[i];
-  eval_f<NS>(P, qj, qj_old, Rj, bx, by, dt, rt, scal_f);
-  double mx = fabs(rt[0]);
-#pragma unroll
-  for (int i = 1; i < NV; ++i) mx = fmax_f(mx, fabs(rt[i]));
-  return mx < NEWTON_TOLF;
-}
-
-// Iteration 1: full Newton step, no line search.  qj receives the iterate.
-template <int NS>
-__device__ bool newton_iter1(const DevParams& P, double* qj, const double* qj_old,
-                             const double* Rj, double bx, double by, double dt,
-                             const double* qj_org, double* qj_rel, double* rt, double& scal_f) {
-  constexpr int NV = 4 + NS;
-  double dd[NV], J2[NV], J3[NV], x_old[NV];
-  newton_direction<NS>(P, bx, by, dt, qj_org, qj_rel, rt, dd, J2, J3);
-#pragma unroll
-  for (int i = 0; i < NV; ++i) x_old[i] = qj_rel[i];
-#pragma unroll
-  for (int i = 0; i < NV; ++i) qj_rel[i] = x_old[i] + dd[i];
-#pragma unroll
-  for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
-  eval_f<NS>(P, qj, qj_old, Rj, bx, by, dt, rt, scal_f);
-#pragma unroll
-  for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
-  return newton_converged<NS>(rt, qj_rel, x_old);
-}
-
-// The residual at the iterate when the previous line search put the old
-// iterate back (rare); true when it already meets TOLF.  Inlined: as a call
-// the iteration pass measured 14.2 against 10.3 ms at 4096^2 (the arrays it
-// takes then live in local memory for the whole pass).
-#ifndef IMEX_RESTART_FN
-#define IMEX_RESTART_FN __device__ __forceinline__
-#endif
-template <int NS>
-IMEX_RESTART_FN bool newton_restart(const DevParams& P, double* qj, const double* qj_old,
-                                    const double* Rj, double bx, double by, double dt,
-                                    const double* qj_org, const double* qj_rel, double* rt,
-                                    double& scal_f) {
-  constexpr int NV = 4 + NS;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
-  eval_f<NS>(P, qj, qj_old, Rj, bx, by, dt, rt, scal_f);
-  double mx = fabs(rt[0]);
-#pragma unroll
-  for (int i = 1; i < NV; ++i) mx = fmax_f(mx, fabs(rt[i]));
-  return mx < NEWTON_TOLF;
-}
-
-// Iterations 2..100: residual at the iterate, Newton direction and lnsrch
-// (src/solver_2d.f90:1815-1824, 1929-1962, 2019-2224).  The reference
-// evaluates the residual at the start of every iteration; it equals the one
-// left by the previous iteration unless that iteration's line search put the
-// old iterate back (alam < alamin or the trial cap), leaving the residual of
-// its last trial: `stale` marks that case and the residual is evaluated
-// again (the loop only continues after such a restore when the relative
-// step is NaN).  Every backtrack after the first halves alam: the cubic
-// model's value is clamped to <= alam/2 and then maxed with alam/2.  The
-// trials are capped at 4096; the cap exits like alam < alamin.
-template <int NS>
-IMEX_FLAT bool newton_iterk(const DevParams& P, double* qj, const double* qj_old,
-                                          const double* Rj, double bx, double by, double dt,
-                                          const double* qj_org, double* qj_rel, double* rt,
-                                          double& scal_f, long long& trials, bool& stale) {
-  constexpr int NV = 4 + NS;
-  if (stale) {
-    stale = false;
-    if (newton_restart<NS>(P, qj, qj_old, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f)) return true;
-  }
-  double dd[NV], J2[NV], J3[NV], x_old[NV];
-  // the later iterations evaluate the Jacobian columns side by side (0.3 ms
-  // per step less at 4096^2 than one column at a time)
-  newton_direction<NS, true>(P, bx, by, dt, qj_org, qj_rel, rt, dd, J2, J3);
-#pragma unroll
-  for (int i = 0; i < NV; ++i) x_old[i] = qj_rel[i];
-  const double scal_f_old = scal_f;
-  double sdot = 0.0;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) sdot += qj_rel[i] * qj_rel[i];
-  double stpmax = NEWTON_STPMX * fmax_f(sqrt(sdot), (double)NV);
-  double grad[NV];
+  double J2[NV], J3[NV];
+  newton_direction<NS>(P, bx, by, dt, in, in + NV, in + 2 * NV, out, J2, J3);
 #pragma unroll
   for (int c = 0; c < NV; ++c) {
     double s = 0.0;
@@ -1520,59 +1410,235 @@ IMEX_FLAT bool newton_iterk(const DevParams& P, double* qj, const double* qj_old
       double L;
       if (c == 1) L = J2[r];
       else if (c == 2) L = J3[r];
-      else L = (r == c) ? 1.0 * qj_org[c] : 0.0;
-      s += rt[r] * L;
+      else L = (r == c) ? 1.0 * in[c] : 0.0;
+      s += in[2 * NV + r] * L;
     }
-    grad[c] = s;
+    out[NV + c] = s;
   }
-  // NORM2(dd) > stpmax scales the step.  The scaled sum below ends with
-  // scale = MAX|dd| and ssq <= NV (each term at most 1) up to a few
-  // roundings, so its result is below 3*MAX|dd| for NV <= 8; when that bound
-  // is already below stpmax (finite), the norm cannot exceed it and is not
-  // evaluated.  A NaN component gives a NaN norm and no scaling either way.
-  static_assert(NV <= 8, "the norm bound 3*MAX|dd| holds for up to 8 components");
-  double dmax = 0.0;
+}
+
+// dd and grad from the friction's imaginary parts nim (friction_jacobian) where
+// `ok` says they hold; with a finite rt of ordinary size the zero rows of
+// the Jacobian add exact zeros and are left out.  Otherwise the general call.
+template <int NS, int ST>
+IMEX_FLAT void newton_dir_grad(const DevParams& P, double bx, double by, double dt,
+                               const double* qj_org, const double* qj_rel, const double* rt,
+                               bool ok, const double* nim, double* dd, double* grad) {
+  constexpr int NV = 4 + NS;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) dmax = fmax_f(dmax, fabs(dd[i]));
-  if (!(3.0 * dmax < stpmax)) {
-    double scale = 0.0, ssq = 0.0;
+  for (int i = 0; i < NV; ++i) ok = ok & below_huge(rt[i]) & below_huge(qj_org[i * ST]);
+  if (ok && dt > 0.0 && dt < 1e300) {
+    const double s11 = 1.0 * qj_org[1 * ST] - dt * 1.0 * (1.0 * nim[0] * P.one_by_h);
+    const double s21 = 0.0 - dt * 1.0 * (1.0 * nim[1] * P.one_by_h);
+    const double s12 = 0.0 - dt * 1.0 * (1.0 * nim[2] * P.one_by_h);
+    const double s22 = 1.0 * qj_org[2 * ST] - dt * 1.0 * (1.0 * nim[3] * P.one_by_h);
+    const double inv_det = 1.0 / (s11 * s22 - s21 * s12);
+    const double sol0 = (rt[1] * s22 - rt[2] * s12) * inv_det;
+    const double sol1 = (s11 * rt[2] - s21 * rt[1]) * inv_det;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      if (dd[i] != 0.0) {
-        double ax = fabs(dd[i]);
-        if (scale < ax) {
-          double val = scale / ax;
-          ssq = 1.0 + ssq * val * val;
-          scale = ax;
-        } else {
-          double val = ax / scale;
-          ssq = ssq + val * val;
+      if (i == 1 || i == 2) continue;
+      dd[i] = 0.0 + (-(rt[i] / (1.0 * qj_org[i * ST])));
+      grad[i] = 0.0 + rt[i] * (1.0 * qj_org[i * ST]);
+    }
+    dd[1] = -sol0 + 0.0;
+    dd[2] = -sol1 + 0.0;
+    grad[1] = (0.0 + rt[1] * s11) + rt[2] * s21;
+    grad[2] = (0.0 + rt[1] * s12) + rt[2] * s22;
+    return;
+  }
+  double in[3 * NV], out[2 * NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    in[i] = qj_org[i * ST];
+    in[NV + i] = qj_rel[i];
+    in[2 * NV + i] = rt[i];
+  }
+  newton_direction_any<NS>(P, bx, by, dt, in, out);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    dd[i] = out[i];
+    grad[i] = out[NV + i];
+  }
+}
+
+// Scaling (src/solver_2d.f90:1786-1798).
+template <int NS>
+__device__ __forceinline__ void newton_scale(const double* qj, double* qj_org) {
+  constexpr int NV = 4 + NS;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) qj_org[i] = fmax_f(fabs(qj[i]), 1.0e-3);
+}
+
+// Before the first iteration: the scaling of the start g, and qj_rel = g/qj_org.
+// The reference's residual test before the first Jacobian is taken at g; where the
+// scaling is exact (g = qj_rel*qj_org, as it is for |g| >= 1e-3) the first
+// newton_step takes it with its Jacobian (need_rt), else it is taken here.  True: g
+// already meets TOLF (nl_iter = 1); the iterate qj_rel*qj_org is then g.
+template <int NS, int ST>
+IMEX_FLAT bool newton_begin(const DevParams& P, const double* g, const double* qj_old,
+                            const double* Rj, double bx, double by, double dt, double* qj_org,
+                            double* qj_rel, double* rt, double& scal_f, bool& need_rt) {
+  constexpr int NV = 4 + NS;
+  bool same = true;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const double org = fmax_f(fabs(g[i]), 1.0e-3);
+    qj_org[i * ST] = org;
+    // g/|g| is +-1
+    const double x =
+        (fabs(g[i]) >= 1.0e-3 && below_huge(g[i])) ? copysign(1.0, g[i]) : g[i] / org;
+    same = same && x * org == g[i];
+    qj_rel[i] = x;
+    rt[i] = 0.0;
+  }
+  scal_f = 0.0;
+  need_rt = same;
+  if (same) return false;
+  double nh2, nh3;
+  friction_any<NS>(P, bx, by, g, nh2, nh3);
+  newton_residual<NS, ST>(g, qj_old, Rj, nh2, nh3, dt, rt, scal_f);
+  double mx = fabs(rt[0]);
+#pragma unroll
+  for (int i = 1; i < NV; ++i) mx = fmax_f(mx, fabs(rt[i]));
+  if (!(mx < NEWTON_TOLF)) return false;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    qj_org[i * ST] = 1.0;
+    qj_rel[i] = g[i];
+  }
+  return true;
+}
+
+// One Newton iteration (src/solver_2d.f90:1815-1824, 1879-1988); qj_rel
+// receives the iterate (times qj_org), rt its residual.  Iteration 1 is a full
+// step; the later ones search along it with lnsrch (:2019-2224).  The
+// reference evaluates the residual at the start of every iteration; it
+// equals the one left by the previous iteration, so it is taken only in iteration 1
+// (need_rt) and where the previous iteration's line search put the old
+// iterate back (alam < alamin or the trial cap), leaving the residual of
+// its last trial: `stale` marks that case (the loop only continues after such a
+// restore when the relative step is NaN).  Every backtrack after the first
+// halves alam: the cubic model's value is clamped to <= alam/2 and then maxed with
+// alam/2.  The trials are capped at 4096; the cap exits like alam < alamin.
+// All iterations share this code, so that a warp in its second or third
+// iteration finds it in the instruction cache.  With *defer set, a cell whose
+// state needs the general direction is left as it is, with *defer still set
+// (cleared otherwise).
+template <int NS, int ST, bool STOP = true>
+IMEX_FLAT bool newton_step(const DevParams& P, bool first, bool need_rt, const double* qj_old,
+                           const double* Rj, const double* qj_org, double bx, double by, double dt,
+                           double* qj_rel, double* rt, double& scal_f, unsigned& trials,
+                           bool& stale, bool* defer = nullptr) {
+  constexpr int NV = 4 + NS;
+  double dd[NV], slope = 0.0;
+  {
+    double x[NV], grad[NV], nh2, nh3, nim[4];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) x[i] = qj_rel[i] * qj_org[i * ST];
+    const bool ok = friction_jacobian<NS, STOP>(P, bx, by, x, P.hstep * qj_org[1 * ST],
+                                                P.hstep * qj_org[2 * ST], nh2, nh3, nim);
+    if (defer && *defer) {
+      *defer = !ok;
+      if (!ok) return false;
+    }
+    if (need_rt || stale) {
+      stale = false;
+      if (!ok) friction_any<NS>(P, bx, by, x, nh2, nh3);
+      newton_residual<NS, ST>(x, qj_old, Rj, nh2, nh3, dt, rt, scal_f);
+      double mx = fabs(rt[0]);
+#pragma unroll
+      for (int i = 1; i < NV; ++i) mx = fmax_f(mx, fabs(rt[i]));
+      if (mx < NEWTON_TOLF) return true;
+    }
+    newton_dir_grad<NS, ST>(P, bx, by, dt, qj_org, qj_rel, rt, ok, nim, dd, grad);
+    // NORM2(dd) > stpmax = STPMX*MAX(NORM2(qj_rel), NV) scales the step.  The
+    // scaled sum below ends with scale = MAX|dd| and ssq <= NV (each term at
+    // most 1) up to a few roundings, so its result is below 3*MAX|dd| for
+    // NV <= 8; when that bound is already below stpmax (finite), or below
+    // STPMX*NV, the norms are not evaluated.  A NaN component gives a NaN norm
+    // and no scaling either way.
+    static_assert(NV <= 8, "the norm bound 3*MAX|dd| holds for up to 8 components");
+    double dmax = 0.0;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) dmax = fmax_f(dmax, fabs(dd[i]));
+    if (!first && !(3.0 * dmax < NEWTON_STPMX * (double)NV)) {
+      double sdot = 0.0;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) sdot += qj_rel[i] * qj_rel[i];
+      const double stpmax = NEWTON_STPMX * fmax_f(sqrt(sdot), (double)NV);
+      if (!(3.0 * dmax < stpmax)) {
+        double scale = 0.0, ssq = 0.0;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          if (dd[i] != 0.0) {
+            double ax = fabs(dd[i]);
+            if (scale < ax) {
+              double val = scale / ax;
+              ssq = 1.0 + ssq * val * val;
+              scale = ax;
+            } else {
+              double val = ax / scale;
+              ssq = ssq + val * val;
+            }
+          }
+        }
+        double dabs = scale * sqrt(ssq);
+        if (dabs > stpmax) {
+#pragma unroll
+          for (int i = 0; i < NV; ++i) dd[i] = dd[i] * stpmax / dabs;
         }
       }
     }
-    double dabs = scale * sqrt(ssq);
-    if (dabs > stpmax) {
 #pragma unroll
-      for (int i = 0; i < NV; ++i) dd[i] = dd[i] * stpmax / dabs;
-    }
+    for (int i = 0; i < NV; ++i) slope += grad[i] * dd[i];
   }
-  double slope = 0.0;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) slope += grad[i] * dd[i];
-  double mx = 0.0;
+  // qj_rel keeps the old iterate until the end of the search
+  bool xfin = true, fin = true;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    double r = fabs(dd[i]) / fmax_f(fabs(x_old[i]), 1.0);
-    mx = (i == 0) ? r : fmax_f(mx, r);
+    xfin = xfin & isfinite(qj_rel[i]);
+    fin = fin & isfinite(dd[i]);
   }
-  double alamin = EPS / mx;
-  bool xfin = true;
+  const double scal_f_old = scal_f;
+  double alamin = 1.0, alam = 1.0;
+  bool keep = true;   // the old iterate stays
+  if (!first) {
+    // MAX of |dd_i|/MAX(|x_i|, 1): one division for the largest |dd|, and one
+    // for each other that could still exceed it (|dd_i| bounds its quotient)
+    double mx = 0.0;
+    bool all = !(xfin && fin);
+    if (!all) {
+      double top = 0.0, d = 1.0;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) xfin &= isfinite(x_old[i]);
-  if (alamin == 0.0) {
+      for (int i = 0; i < NV; ++i) {
+        const double a = fabs(dd[i]);
+        if (i == 0 || a > top) {
+          top = a;
+          d = fmax_f(fabs(qj_rel[i]), 1.0);
+        }
+      }
+      mx = (d == 1.0) ? top : top / d;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) qj_rel[i] = x_old[i];
-  } else {
+      for (int i = 0; i < NV; ++i) all |= fabs(dd[i]) > mx;
+    }
+    if (all) {
+#pragma unroll 1
+      for (int i = 0; i < NV; ++i) {
+        double a = dd[0], x = qj_rel[0];
+#pragma unroll
+        for (int m = 1; m < NV; ++m)
+          if (m == i) {
+            a = dd[m];
+            x = qj_rel[m];
+          }
+        const double r = fabs(a) / fmax_f(fabs(x), 1.0);
+        mx = (i == 0) ? r : fmax_f(mx, r);
+      }
+    }
+    alamin = EPS / mx;
+  }
+  if (alamin != 0.0) {
     // Rows other than 2, 3 carry no implicit term: eval_f's sum of f^2
     // taken over them alone, in eval_f's order, cannot exceed the full sum
     // (rounded addition of a term >= 0 never decreases a sum, and rounding
@@ -1587,29 +1653,35 @@ IMEX_FLAT bool newton_iterk(const DevParams& P, double* qj, const double* qj_old
     // After the first backtrack every alam is half the previous one,
     // whatever a trial's outcome, so two consecutive trials' partial sums
     // are evaluated side by side (independent chains) and their outcomes
-    // then taken in order, as one trial after the other.
-    auto partial_half_sum = [&](double al) {
+    // then taken in order, as one trial after the other.  Once a trial leaves
+    // all those rows' iterates where they were (x + alam*dd rounds to x, as
+    // it then does for every smaller alam), the partial sum no longer changes:
+    // the remaining trials fail with it and are only counted.
+    auto partial_half_sum = [&](double al, bool& still) {
       double d = 0.0;
+      still = true;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
         if (i == 1 || i == 2) continue;
-        const double qt = (x_old[i] + al * dd[i]) * qj_org[i];
-        const double R = Rj[i] - 1.0 * 0.0;
-        const double fi = qt - qj_old[i] + dt * R;
+        const double xo = qj_rel[i], xt = xo + al * dd[i];
+        still = still & (xt == xo);
+        const double qt = xt * qj_org[i * ST];
+        const double R = Rj[i * ST] - 1.0 * 0.0;
+        const double fi = qt - qj_old[i * ST] + dt * R;
         const double f = 1.0 * fi;
         d += f * f;
       }
       return 0.5 * d;
     };
     const double sf_thr = 0.9 * scal_f_old;
-    double alam = 1.0;
     int trial = 0;
     bool capped = true;   // the loop ran out of its 4096 trials
     while (trial < 4096) {
       if (trial > 0 && alam != 1.0 && xfin) {
         const double alam_b = 0.5 * alam;
-        const double ha = partial_half_sum(alam);
-        const double hb = partial_half_sum(alam_b);
+        bool still_a, still_b;
+        const double ha = partial_half_sum(alam, still_a);
+        const double hb = partial_half_sum(alam_b, still_b);
         if (ha > sf_thr) {            // trial `trial` fails
           ++trials;
           if (alam < alamin) {
@@ -1620,14 +1692,19 @@ IMEX_FLAT bool newton_iterk(const DevParams& P, double* qj, const double* qj_old
           alam = alam_b;
           if (++trial >= 4096) break;
           if (alam != 1.0 && hb > sf_thr) {   // and so does the next one
-            ++trials;
-            if (alam < alamin) {
-              capped = false;
-              stale = true;
-              break;
-            }
-            alam = 0.5 * alam;
-            ++trial;
+            bool out = false;
+            do {                              // (and, still_b, all after it)
+              ++trials;
+              if (alam < alamin) {
+                capped = false;
+                stale = true;
+                out = true;
+                break;
+              }
+              alam = 0.5 * alam;
+              ++trial;
+            } while (still_b && trial < 4096);
+            if (out) break;
             continue;
           }
         }
@@ -1635,20 +1712,20 @@ IMEX_FLAT bool newton_iterk(const DevParams& P, double* qj, const double* qj_old
       // a trial with the full residual
       double qt[NV];
 #pragma unroll
-      for (int i = 0; i < NV; ++i) qj_rel[i] = x_old[i] + alam * dd[i];
-#pragma unroll
-      for (int i = 0; i < NV; ++i) qt[i] = qj_rel[i] * qj_org[i];
-      eval_f<NS>(P, qt, qj_old, Rj, bx, by, dt, rt, scal_f);
-      ++trials;
-      if (scal_f <= sf_thr) {
-        capped = false;
-        break;
+      for (int i = 0; i < NV; ++i) {
+        const double xt = qj_rel[i] + alam * dd[i];
+        qt[i] = xt * qj_org[i * ST];
       }
+      eval_f<NS, ST>(P, qt, qj_old, Rj, bx, by, dt, rt, scal_f);
+      capped = false;
+      if (first) break;
+      ++trials;
+      if (scal_f <= sf_thr) break;
       if (alam < alamin) {
-        capped = false;
         stale = true;
         break;
       }
+      capped = true;
       if (alam == 1.0) {
         double tmplam = -slope / (2.0 * (scal_f - scal_f_old - slope));
         alam = fmax_f(tmplam, 0.5 * alam);
@@ -1657,17 +1734,32 @@ IMEX_FLAT bool newton_iterk(const DevParams& P, double* qj, const double* qj_old
       }
       ++trial;
     }
-    if (stale || capped) {
-      // alam < alamin or the trial cap: the old iterate is put back
-#pragma unroll
-      for (int i = 0; i < NV; ++i) qj_rel[i] = x_old[i];
+    // alam < alamin or the trial cap: the old iterate is put back
+    keep = stale || capped;
+    if (keep) {
       scal_f = scal_f_old;
       stale = true;
     }
   }
+  // the exit tests (src/solver_2d.f90:1964-1988): MAX|rt| < TOLF, or
+  // MAX over i of |x_i - x_old_i|/MAX(|x_i|, 1) < EPS.  MAX skips NaN
+  // quotients (all NaN: NaN, and the test fails), so the second holds when
+  // some quotient is a number and every such quotient is below EPS; each
+  // comparison of a rounded quotient is taken without the division where
+  // its answer is certain (rel_change_below).
+  bool any = false, below = true;
+  double mx = fabs(rt[0]);
 #pragma unroll
-  for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
-  return newton_converged<NS>(rt, qj_rel, x_old);
+  for (int i = 0; i < NV; ++i) {
+    if (i > 0) mx = fmax_f(mx, fabs(rt[i]));
+    const double xo = qj_rel[i], x = keep ? xo : xo + alam * dd[i];
+    qj_rel[i] = x;
+    const double d = fabs(x - xo), s = fmax_f(fabs(x), 1.0);
+    if (isnan(d) || (isinf(d) && isinf(s))) continue;   // the quotient is NaN
+    any = true;
+    below = below & rel_change_below(d, s, EPS);
+  }
+  return mx < NEWTON_TOLF || (any && below);
 }
 
 // ============================================================ mass exchange
@@ -1838,20 +1930,19 @@ __device__ bool erosion_cell(const DevParams& P, double* qc, double bx, double b
 }
 
 // =============================================================== stage 2
-// RK stage 2 (src/solver_2d.f90:1105-1628) as passes over the solve cells:
-//   k_stage2_first   q_fv, semi-implicit terms, q_si, Rj_not_impl, Newton
-//                    scaling and iteration 1; cells that go on are appended
-//                    to list 0
-//   k_stage2_iter    one Newton iteration (nl_iter = 2 or 3) over a list;
-//                    cells that go on are appended to the next list
-//   k_stage2_tail    iterations 4..100 for the few cells still iterating
-//   k_stage2_post    sign guard, assemble_sol checks and fixes, q written
-// Between passes a cell's Newton state (qj_rel, the residual, its norm) is
+// RK stage 2 (src/solver_2d.f90:1105-1628):
+//   k_stage2         q_fv, semi-implicit terms, q_si, Rj_not_impl, the Newton
+//                    solve, sign guard, assemble_sol checks and fixes, q
+//                    written: one thread per cell, its vectors in shared memory
+//   k_stage2_rest    on large grids, the cells that k_stage2 left iterating
+//                    when few lanes of their warp were, compacted in a list
+// With the learned start or its harvest the solve is cut where those need it:
+// k_stage2_first (up to iteration 1, or to the network's inputs), the network and
+// k_stage2_wstart, k_stage2_rest over the list of the cells still iterating,
+// k_stage2_post (sign guard and assembly).
+// Between kernels a cell's Newton state (qj_rel, the residual, its norm) is
 // kept in the NewtonWork planes; the iterate is carried bit for bit, so a
-// cell's arithmetic is that of one uninterrupted solve_rk_step.  Iteration
-// counts differ from cell to cell (mostly 2 or 3 here); running each
-// iteration as its own pass over the cells that need it keeps a warp's
-// lanes on the same iteration.
+// cell's arithmetic is that of one uninterrupted solve_rk_step.
 struct NewtonWork {
   double* qsi;    // nv planes: q_si, the Newton initial guess (scaling source)
   double* Rj;     // nv planes: Rj_not_impl
@@ -1859,8 +1950,9 @@ struct NewtonWork {
   double* rt;     // nv planes: residual
   double* sf;     // 1 plane: 0.5*|residual|^2
   uint8_t* status;  // 1 plane: bit 0 the cell went through Newton, bit 1 its
-                    // residual must be evaluated again (see newton_iterk)
-  uint32_t* list[3];  // cells (k*pitch + j) still iterating after pass 0, 1, 2
+                    // residual must be evaluated again (see newton_step); listed
+                    // cells: iterations taken in the upper bits
+  uint32_t* list;   // cells (k*pitch + j) still iterating
   // learned warm start (warm != 0): the Newton cells of the step, their
   // network inputs and the network's momentum guesses
   int warm;
@@ -1925,37 +2017,40 @@ __device__ __forceinline__ unsigned int list_append(bool add, uint32_t c, uint32
   return add ? slot : 0xffffffffu;
 }
 
-// Newton statistics of the cells that finished in this warp iteration
-// (iters = 0: no cell finished in this lane).
-__device__ __forceinline__ void newton_finish_stats(DevClock* clk, int iters,
-                                                    unsigned long long& it_sum,
-                                                    unsigned long long& maxit) {
+// Newton statistics of a block (or warp), summed in shared memory and added to
+// the clock at its end by threads t = 0..: one global atomic per warp and
+// counter queued a few million of them on one address at 4096^2.
+struct NewtonStats {
+  unsigned hist[16];
+  unsigned long long cells, iters, trials, maxit;
+};
+__device__ __forceinline__ void stat_reset(NewtonStats& S, int t) {   // a barrier must follow
+  if (t < 16) S.hist[t] = 0;
+  if (t == 16) S.cells = S.iters = S.trials = S.maxit = 0;
+}
+// One warp's cells: `cell` took part, finished after `iters` iterations (0: not
+// finished here), with `trials` line-search trials.
+__device__ __forceinline__ void stat_add(NewtonStats& S, bool cell, int iters, unsigned trials) {
   const int bin = iters > 0 ? (iters < 16 ? iters - 1 : 15) : -1;
   const unsigned peers = __match_any_sync(0xffffffffu, bin);
-  if (bin >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1)
-    atomicAdd(&clk->hist[bin], (unsigned long long)__popc(peers));
-  if (iters > 0) {
-    it_sum += (unsigned long long)iters;
-    if (iters >= NEWTON_MAX_IT) maxit += 1;
+  if (bin >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&S.hist[bin], __popc(peers));
+  const unsigned n = __popc(__ballot_sync(0xffffffffu, cell));
+  const unsigned full = __popc(__ballot_sync(0xffffffffu, iters >= NEWTON_MAX_IT));
+  const unsigned it = __reduce_add_sync(0xffffffffu, (unsigned)iters);
+  const unsigned tr = __reduce_add_sync(0xffffffffu, trials);
+  if ((threadIdx.x & 31) == 0) {
+    if (n) atomicAdd(&S.cells, (unsigned long long)n);
+    if (it) atomicAdd(&S.iters, (unsigned long long)it);
+    if (tr) atomicAdd(&S.trials, (unsigned long long)tr);
+    if (full) atomicAdd(&S.maxit, (unsigned long long)full);
   }
 }
-
-__device__ __forceinline__ void newton_flush_stats(DevClock* clk, unsigned long long cells,
-                                                   unsigned long long it_sum,
-                                                   unsigned long long trials,
-                                                   unsigned long long maxit) {
-  for (int off = 16; off > 0; off >>= 1) {
-    cells += __shfl_down_sync(0xffffffffu, cells, off);
-    it_sum += __shfl_down_sync(0xffffffffu, it_sum, off);
-    trials += __shfl_down_sync(0xffffffffu, trials, off);
-    maxit += __shfl_down_sync(0xffffffffu, maxit, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (cells) atomicAdd(&clk->newton_cells, cells);
-    if (it_sum) atomicAdd(&clk->newton_iters, it_sum);
-    if (trials) atomicAdd(&clk->lnsrch_trials, trials);
-    if (maxit) atomicAdd(&clk->newton_maxit, maxit);
-  }
+__device__ __forceinline__ void stat_flush(const NewtonStats& S, DevClock* clk, int t) {   // after a barrier
+  if (t < 16 && S.hist[t]) atomicAdd(&clk->hist[t], (unsigned long long)S.hist[t]);
+  if (t == 16 && S.cells) atomicAdd(&clk->newton_cells, S.cells);
+  if (t == 17 && S.iters) atomicAdd(&clk->newton_iters, S.iters);
+  if (t == 18 && S.trials) atomicAdd(&clk->lnsrch_trials, S.trials);
+  if (t == 19 && S.maxit) atomicAdd(&clk->newton_maxit, S.maxit);
 }
 
 template <int NS>
@@ -1964,6 +2059,24 @@ __device__ __forceinline__ bool all_finite(const double* v) {
 #pragma unroll
   for (int i = 0; i < 4 + NS; ++i) ok &= isfinite(v[i]);
   return ok;
+}
+
+// Newton iterations `it`.. of a cell until it ends (100 at most); returns the
+// last iteration's number, `done` whether it converged.
+template <int NS, int ST>
+IMEX_FLAT int newton_finish(const DevParams& P, int it, bool need_rt, const double* qj_old,
+                            const double* Rj, const double* qj_org, double bx, double by, double dt,
+                            double* qj_rel, double* rt, double& scal_f, unsigned& trials,
+                            bool& stale, bool& done) {
+  done = false;
+#pragma unroll 1
+  for (; it <= NEWTON_MAX_IT; ++it) {
+    done = newton_step<NS, ST>(P, it == 1, need_rt, qj_old, Rj, qj_org, bx, by, dt, qj_rel, rt,
+                               scal_f, trials, stale);
+    need_rt = false;
+    if (done) break;
+  }
+  return it > NEWTON_MAX_IT ? NEWTON_MAX_IT : it;
 }
 
 // Fallback of a warm start that failed (no convergence in 100 iterations, or
@@ -1977,112 +2090,484 @@ __device__ __forceinline__ int newton_plain(const DevParams& P, const NewtonWork
   constexpr int NV = 4 + NS;
   const size_t N = (size_t)P.plane;
   double qj_org[NV], qj_rel[NV], rt[NV], scal_f;
+  bool need_rt, stale = false, done;
+  int it = 1;
+  unsigned tr = 0;
 #pragma unroll
   for (int i = 0; i < NV; ++i) qj[i] = W.qsi[c + i * N];
-  newton_scale<NS>(qj, qj_org);
-  if (newton_start<NS>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f)) return 1;
-  if (newton_iter1<NS>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f)) return 1;
-  bool stale = false;
-  int it;
-  for (it = 2; it <= NEWTON_MAX_IT; ++it) {
-    long long tr = 0;
-    bool done = newton_iterk<NS>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f, tr, stale);
-    trials += (unsigned long long)tr;
-    if (done) break;
-  }
-  return it > NEWTON_MAX_IT ? NEWTON_MAX_IT : it;
+  if (!newton_begin<NS, 1>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f, need_rt))
+    it = newton_finish<NS, 1>(P, 1, need_rt, q0, Rj, qj_org, bx, by, dt, qj_rel, rt, scal_f, tr,
+                              stale, done);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
+  trials += tr;
+  return it;
 }
 
-// Stage 2 up to Newton iteration 1 for one lane's cell (plane index c; the
-// lane takes part in the warp's list appends whether or not it has a cell).
+// Stage 2 before the Newton solve of the cell with old state q0 and stage-1
+// tendency Xc: q_fv, the semi-implicit terms, q_si and Rj_not_impl.  False: no
+// solve (q_fv(1) <= 0), qsi receives q_fv.
 template <int NS>
-__device__ __forceinline__ void stage2_first_lane(
-    const DevParams& P, const double* __restrict__ q, const double* __restrict__ X,
-    const uint8_t* __restrict__ mask, const double* __restrict__ Bx,
-    const double* __restrict__ By, const double* __restrict__ Bxx,
-    const double* __restrict__ Bxy, const double* __restrict__ Byy,
-    const double* __restrict__ gc, NewtonWork W, DevClock* clk, double dt, bool valid,
-    size_t c, unsigned long long& cells, unsigned long long& it_sum,
-    unsigned long long& maxit) {
+IMEX_FLAT bool stage2_start(const DevParams& P, const double* q0, const double* Xc, size_t c,
+                            const double* __restrict__ Bx, const double* __restrict__ By,
+                            const double* __restrict__ Bxx, const double* __restrict__ Bxy,
+                            const double* __restrict__ Byy, const double* __restrict__ gc,
+                            double dt, double* qsi, double* Rj, double& bx, double& by) {
   constexpr int NV = 4 + NS, NP = 6 + NS;
+  double qfv[NV];
+  // q_fv = q0 - dt*(MATMUL(divFlux-expl, a_tilde) - MATMUL(NH+SI_NH, a_dirk))
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    double sa = (0.0 + Xc[i] * 1.0) + (0.0 - 0.0) * 0.0;
+    double sb = (0.0 + (0.0 + 0.0) * 0.0) + (0.0 + 0.0) * 0.0;
+    qfv[i] = q0[i] - dt * (sa - sb);
+    qsi[i] = qfv[i];
+    Rj[i] = 0.0;
+  }
+  bx = by = 0.0;
+  if (!(qfv[0] > 0.0)) return false;
+  double qpv[NP];
+  qc_to_qp<NS>(P, qfv, qpv);
+  bx = Bx[c];
+  by = By[c];
+  double bxx = 0.0, bxy = 0.0, byy = 0.0, gcf = 1.0;
+  if (P.curvature_term_flag) {
+    bxx = Bxx[c];
+    bxy = Bxy[c];
+    byy = Byy[c];
+  }
+  if (P.slope_correction_flag) gcf = gc[c];
+  double si2, si3;
+  semi_impl_terms<NS>(P, bx, by, bxx, bxy, byy, gcf, qpv, si2, si3);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const double SI = (i == 1) ? si2 : ((i == 2) ? si3 : 0.0);
+    qsi[i] = qfv[i] + dt * 1.0 * SI;
+  }
+  if (qfv[1] * qfv[1] + qfv[2] * qfv[2] == 0.0) {
+    qsi[1] = 0.0;
+    qsi[2] = 0.0;
+  } else if (qsi[1] * qfv[1] < 0.0 || qsi[2] * qfv[2] < 0.0) {
+    qsi[1] = 0.0;
+    qsi[2] = 0.0;
+  } else {
+    double Sm = sqrt(qsi[1] * qsi[1] + qsi[2] * qsi[2]);
+    double Fm = sqrt(qfv[1] * qfv[1] + qfv[2] * qfv[2]);
+    qsi[1] = Sm * qfv[1] / Fm;
+    qsi[2] = Sm * qfv[2] / Fm;
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    // rows other than 2, 3: qsi = qfv + dt*0 (or +0 for qfv = -0), so
+    // for finite qfv and a finite dt > 0 the difference is +0 and so
+    // is the quotient
+    double SI;
+    if (i != 1 && i != 2 && isfinite(qfv[i]) && dt > 0.0 && dt < 1e300) SI = 0.0;
+    else SI = (qsi[i] - qfv[i]) / (dt * 1.0);
+    double sa = 0.0 + Xc[i] * 1.0;
+    double sb = 0.0 + (0.0 + 0.0) * 0.0;
+    Rj[i] = (sa - sb) - 1.0 * SI;
+  }
+  return true;
+}
+
+// Sign guard after Newton (src/solver_2d.f90:1238-1255) and assemble_sol
+// (src/solver_2d.f90:1339-1626) of one cell: qc the solve's result (newton: it
+// went through Newton from q_si's momenta qs1, qs2), written to q.
+template <int NS>
+IMEX_FLAT void stage2_assemble(const DevParams& P, double* qc, bool newton, double qs1, double qs2,
+                               double* __restrict__ q, const uint8_t* __restrict__ cellinfo,
+                               DevClock* clk, int j, int k) {
+  constexpr int NV = 4 + NS, NP = 6 + NS;
+  const int nx = P.nx, ny = P.ny;
   const size_t N = (size_t)P.plane;
-  bool go_on = false, warm_cell = false;
+  const size_t c = (size_t)k * P.pitch + j;
+  if (newton) {
+    if (ny == 1) qc[2] = 0.0;
+    if (nx == 1) qc[1] = 0.0;
+    if (qs1 * qs1 + qs2 * qs2 == 0.0) {
+      qc[1] = 0.0;
+      qc[2] = 0.0;
+    } else if (qc[1] * qs1 <= 0.0 && qc[2] * qs2 <= 0.0) {
+      qc[1] = 0.0;
+      qc[2] = 0.0;
+    } else {
+      double Sm = sqrt(qc[1] * qc[1] + qc[2] * qc[2]);
+      double Fm = sqrt(qs1 * qs1 + qs2 * qs2);
+      qc[1] = Sm * qs1 / Fm;
+      qc[2] = Sm * qs2 / Fm;
+    }
+  }
+  const long long cell = (long long)k * nx + j;
+  bool anynan = false;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) anynan |= isnan(qc[i]);
+  if (anynan) record_error(clk, 1, cell);
+  if (qc[0] < EPS) {
+    if (qc[0] > -1.0e-7) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) qc[i] = 0.0;
+    } else {
+      record_error(clk, 2, cell);
+    }
+  }
+  bool anyneg = false, anybad = false;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) anyneg |= (qc[4 + i] < 0.0);
+  if (anyneg) {
+#pragma unroll
+    for (int i = 0; i < NS; ++i) anybad |= (qc[4 + i] <= -1.0e-7);
+    if (anybad) {
+      record_error(clk, 3, cell);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NS; ++i)
+        if (qc[4 + i] > -1.0e-7) qc[4 + i] = 0.0;
+    }
+  }
+  double qpv[NP];
+  qc_to_qp<NS>(P, qc, qpv);
+  if (qpv[3] < 273.0) record_error(clk, 4, cell);
+  double ssum = 0.0;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) ssum += qc[4 + i];
+  if (ssum > qc[0]) {
+    if ((ssum - qc[0]) / qc[0] < 1.0e-10 || qc[0] < EPS) {
+      double s = 0.0;
+#pragma unroll
+      for (int i = 0; i < NS; ++i) s += qc[4 + i];
+#pragma unroll
+      for (int i = 0; i < NS; ++i) qc[4 + i] = qc[4 + i] / s * qc[0];
+    } else {
+      record_error(clk, 5, cell);
+    }
+  }
+  if (P.has_cellinfo && (cellinfo[cell] & CI_NODATA)) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) qc[i] = 0.0;
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) q[c + i * N] = qc[i];
+}
+
+// The vectors that live through a cell's solve, one column per thread.  In
+// registers they and the solve's temporaries spilled (at 80 registers 300
+// local accesses per cell, whose lines reached DRAM: 588 MB written by the
+// former first pass for 237 MB of results).
+template <int NS, int T>
+struct NewtonShared {
+  double q0[4 + NS][T], Rj[4 + NS][T], org[4 + NS][T];
+  double qs[2][T];   // q_si's momenta
+  NewtonStats st;
+};
+
+// Steps with at least this many solve cells leave some cells to the compacted
+// list of k_stage2_rest (LIST): those that the lean Jacobian does not cover
+// (the rest's code evicts the others', see k_stage2: 2.03+0.07 against 3.24 ms
+// on 2048^2 cells of the fractal workload, 0.55+0.05 against 0.75 on 1024^2,
+// equal on 512^2), and a warp's last few iterating lanes.  Below, the
+// list costs more than it saves (160 thousand solve cells of a 1024^2 grid:
+// 0.235+0.036 ms with it, 0.207 without; on a slope 0.28 and 0.09 ms).
+constexpr unsigned long long LIST_MIN_CELLS = 1 << 18;
+// Lanes still iterating at or below which a warp leaves them to the list: going on
+// costs the whole warp an iteration, the list about sixty loads and stores per
+// cell (2: 2.05 ms, 6: 2.27 ms, 12: 2.29 ms in the first example above).
+#ifndef IMEX_REST_LANES
+#define IMEX_REST_LANES 2
+#endif
+
+// Stage 2 of one lane's cell (j, k) (the lane takes part in the warp's votes and
+// list appends whether or not it has a solve cell).  LIST: see LIST_MIN_CELLS; both
+// forms in one kernel, chosen per step, spilled twice as much and were slower
+// than either (2.11 ms, 0.045 ms against 0.042 on 100x68 cells).
+template <int NS, int T, bool LIST>
+__device__ __forceinline__ void stage2_lane(
+    const DevParams& P, NewtonShared<NS, T>& S, double* __restrict__ q, const double* __restrict__ X,
+    const uint8_t* __restrict__ mask, const uint8_t* __restrict__ cellinfo,
+    const double* __restrict__ Bx, const double* __restrict__ By, const double* __restrict__ Bxx,
+    const double* __restrict__ Bxy, const double* __restrict__ Byy, const double* __restrict__ gc,
+    const NewtonWork& W, DevClock* clk, double dt, bool valid, int j, int k) {
+  constexpr int NV = 4 + NS, ST = T;
+  const size_t N = (size_t)P.plane;
+  const size_t c = valid ? (size_t)k * P.pitch + j : 0;
+  const bool solve = valid && mask[c];
+  if (!__syncthreads_or(solve)) return;
+  double* q0 = &S.q0[0][threadIdx.x];
+  double* Rj = &S.Rj[0][threadIdx.x];
+  double* org = &S.org[0][threadIdx.x];
+  double rel[NV], rt[NV], scal_f = 0.0, bx = 0.0, by = 0.0;
+  bool newton = false, go = false, need_rt = false, stale = false;
+  int it = 0;   // iterations taken
+  unsigned trials = 0;
+  if (solve) {
+    double qsi[NV];
+    {
+      double qo[NV], Xc[NV], R[NV];
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        qo[i] = q[c + i * N];
+        Xc[i] = X[c + i * N];
+      }
+      newton = stage2_start<NS>(P, qo, Xc, c, Bx, By, Bxx, Bxy, Byy, gc, dt, qsi, R, bx, by);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        q0[i * ST] = qo[i];
+        Rj[i * ST] = R[i];
+      }
+    }
+    if (newton) {
+      S.qs[0][threadIdx.x] = qsi[1];
+      S.qs[1][threadIdx.x] = qsi[2];
+      go = !newton_begin<NS, ST>(P, qsi, q0, Rj, bx, by, dt, org, rel, rt, scal_f, need_rt);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        org[i * ST] = 1.0;
+        rel[i] = qsi[i];
+      }
+    }
+  }
+  bool listed = false;
+#pragma unroll 1
+  for (int n = 1; n <= NEWTON_MAX_IT; ++n) {   // n: this iteration, the same in all lanes
+    // the block's warps go through the iterations together: they then fetch the
+    // same instructions at the same time
+    if (!__syncthreads_or(go)) break;
+    if (LIST && n > 2 && n <= 60 && __popc(__ballot_sync(0xffffffffu, go)) <= IMEX_REST_LANES) {
+      listed = listed || go;
+      go = false;
+    }
+    if (go) {
+      bool defer = LIST && n <= 60;
+      go = !newton_step<NS, ST, !LIST>(P, n == 1, need_rt, q0, Rj, org, bx, by, dt, rel, rt, scal_f,
+                                trials, stale, LIST ? &defer : nullptr);
+      if (defer) {
+        // the list takes it from here (its first residual too, if still to do)
+        listed = true;
+        go = false;
+        stale = stale || need_rt;
+      } else {
+        it = n;
+      }
+      need_rt = false;
+    }
+  }
+  stat_add(S.st, newton, newton && !listed ? max(it, 1) : 0, trials);
+  if (LIST) {
+    list_append(listed, (uint32_t)c, W.list, &clk->nw_count[0]);
+    if (listed) {
+      // q_si's momenta and, for the other rows, their scaling (all >= 1e-3, so
+      // the scaling of these values is itself)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        W.qsi[c + i * N] = (i == 1 || i == 2) ? S.qs[i - 1][threadIdx.x] : org[i * ST];
+        W.Rj[c + i * N] = Rj[i * ST];
+        W.x[c + i * N] = rel[i];
+        W.rt[c + i * N] = rt[i];
+      }
+      W.sf[c] = scal_f;
+      W.status[c] = (uint8_t)((it << 2) | (stale ? 3 : 1));
+    }
+  }
+  if (solve && !listed) {
+    double qc[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) qc[i] = rel[i] * org[i * ST];
+    stage2_assemble<NS>(P, qc, newton, newton ? S.qs[0][threadIdx.x] : 0.0,
+                        newton ? S.qs[1][threadIdx.x] : 0.0, q, cellinfo, clk, j, k);
+  }
+}
+
+// Stage 2 over the grid rows [k0, k1), of the steps whose number of solve cells
+// asks for LIST (the other kernel returns at once): blocks of T threads, 512
+// per SM, at 128 registers (84 registers spilled 2 kB per thread and measured 2.58
+// against 2.04 ms on 2048^2 cells).
+// What bounds it is instruction fetch: the solve's code is larger than the
+// instruction cache, and warps at different places in it evict each other's
+// (1024^2 cells of the fractal workload, warps on their own: 54% hits, 7 of 15
+// stall cycles without an instruction).  So the warps of a block take each
+// phase together, and with LIST, where there is work for it, one block of 512
+// fills the SM: 2.03 ms on 2048^2 cells against 2.18 ms in blocks of 128,
+// which the smaller steps take (a 1024^2 grid with 15% wet cells 0.18 against
+// 0.23 ms).  Rolled Jacobian columns (2.14 ms), a state machine with one
+// place for residuals (2.34 ms) and 160 registers less spill (2.01 ms, but
+// 0.060 against 0.043 ms on 99x99) were no better.
+// The kernels that this replaces, one pass per Newton iteration over lists in
+// memory, took 3.55 ms on those 2048^2 cells, 0.281 ms on that 1024^2 grid (0.269
+// now) and 0.234 on a 301x517 slope (0.088).
+template <int NS, int T, bool LIST>
+__global__ void __launch_bounds__(T, 512 / T)
+    k_stage2(const __grid_constant__ DevParams Pp, double* __restrict__ q,
+             const double* __restrict__ X, const uint8_t* __restrict__ mask,
+             const uint8_t* __restrict__ cellinfo, const double* __restrict__ Bx,
+             const double* __restrict__ By, const double* __restrict__ Bxx,
+             const double* __restrict__ Bxy, const double* __restrict__ Byy,
+             const double* __restrict__ gc, const __grid_constant__ NewtonWork W, DevClock* clk,
+             int k0, int k1, unsigned long long list_min) {
+  const DevParams& P = Pp;
+  if ((clk->solve_cells >= list_min) != LIST) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  NewtonShared<NS, T>& S = *reinterpret_cast<NewtonShared<NS, T>*>(smem_raw);
+  const int nx = P.nx;
+  const long long ncell = (long long)nx * (k1 - k0);
+  const double dt = clk->dt;
+  stat_reset(S.st, threadIdx.x);
+  __syncthreads();
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long base = (long long)blockIdx.x * blockDim.x; base < ncell; base += stride) {
+    const long long g = base + threadIdx.x;
+    stage2_lane<NS, T, LIST>(P, S, q, X, mask, cellinfo, Bx, By, Bxx, Bxy, Byy, gc, W, clk, dt,
+                             g < ncell, (int)(g % nx), k0 + (int)(g / nx));
+  }
+  __syncthreads();
+  stat_flush(S.st, clk, threadIdx.x);
+}
+
+// The remaining iterations of entry e of the list (valid: e is inside the
+// list).  `assemble`: sign guard and assembly follow here (k_stage2's cells), else
+// the result goes to W.x.
+template <int NS>
+__device__ __forceinline__ void stage2_rest_lane(const DevParams& P, double* __restrict__ q,
+                                                 const uint8_t* __restrict__ cellinfo,
+                                                 const double* __restrict__ Bx,
+                                                 const double* __restrict__ By,
+                                                 const NewtonWork& W, DevClock* clk, double dt,
+                                                 bool valid, long long e, bool assemble,
+                                                 NewtonStats& st) {
+  constexpr int NV = 4 + NS;
+  const size_t N = (size_t)P.plane;
   int fin = 0;
-  float fw[WARM_IN];
+  bool fb = false;
+  uint32_t c = 0;
+  unsigned tr = 0;
   if (valid) {
-      if (mask[c]) {
-        double q0[NV], qfv[NV], Xc[NV];
+    c = W.list[e];
+    double q0[NV], Rj[NV], qj_org[NV], qj_rel[NV], rt[NV], qj[NV], scal_f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      q0[i] = q[c + i * N];
+      Rj[i] = W.Rj[c + i * N];
+      qj[i] = W.qsi[c + i * N];
+      qj_rel[i] = W.x[c + i * N];
+      rt[i] = W.rt[c + i * N];
+    }
+    const double qs1 = qj[1], qs2 = qj[2];
+    if (W.warm) {   // the Newton start (scaling source) was the network's guess
+      qj[1] = W.guess[c];
+      qj[2] = W.guess[c + N];
+    }
+    scal_f = W.sf[c];
+    const int status = W.status[c];
+    bool stale = (status & 2) != 0, done;
+    newton_scale<NS>(qj, qj_org);
+    fin = newton_finish<NS, 1>(P, (status >> 2) + 1, false, q0, Rj, qj_org, Bx[c], By[c], dt, qj_rel,
+                               rt, scal_f, tr, stale, done);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
+    if (assemble) {
+      stage2_assemble<NS>(P, qj, true, qs1, qs2, q, cellinfo, clk, (int)(c % P.pitch),
+                          (int)(c / P.pitch));
+    } else {
+      fb = W.warm && (!done || !all_finite<NS>(qj));
+      W.status[c] = 1;
+      if (!fb) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) W.x[c + i * N] = qj[i];
+      }
+    }
+  }
+  stat_add(st, false, fin, tr);
+  if (W.warm) list_append(fb, c, W.flist, &clk->nw_fb);
+}
+
+#ifndef IMEX_REST_MINB
+#define IMEX_REST_MINB 4
+#endif
+template <int NS>
+__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
+    k_stage2_rest(const __grid_constant__ DevParams Pp, double* __restrict__ q,
+                  const uint8_t* __restrict__ cellinfo, const double* __restrict__ Bx,
+                  const double* __restrict__ By, const __grid_constant__ NewtonWork W,
+                  DevClock* clk, int assemble) {
+  __shared__ NewtonStats st;
+  const long long n = (long long)clk->nw_count[0];
+  if ((long long)blockIdx.x * blockDim.x >= n) return;
+  stat_reset(st, threadIdx.x);
+  __syncthreads();
+  const double dt = clk->dt;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n;
+       base += stride) {
+    const long long e = base + (threadIdx.x & 31);
+    stage2_rest_lane<NS>(Pp, q, cellinfo, Bx, By, W, clk, dt, e < n, e, assemble != 0, st);
+  }
+  __syncthreads();
+  stat_flush(st, clk, threadIdx.x);
+}
+
+// Stage 2 up to Newton iteration 1, or with the learned start up to the
+// network's inputs, keeping q_si, Rj and the Newton state in the NewtonWork
+// planes.
+#ifndef IMEX_FIRST_MINB
+#define IMEX_FIRST_MINB 5
+#endif
+template <int NS>
+__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_FIRST_MINB)
+    k_stage2_first(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
+                   const double* __restrict__ X, const uint8_t* __restrict__ mask,
+                   const double* __restrict__ Bx, const double* __restrict__ By,
+                   const double* __restrict__ Bxx, const double* __restrict__ Bxy,
+                   const double* __restrict__ Byy, const double* __restrict__ gc,
+                   const __grid_constant__ NewtonWork W, DevClock* clk) {
+  const DevParams& P = Pp;
+  constexpr int NV = 4 + NS;
+  __shared__ NewtonStats st;
+  const int nx = P.nx;
+  const long long ncell = (long long)nx * P.ny;
+  const size_t N = (size_t)P.plane;
+  const double dt = clk->dt;
+  stat_reset(st, threadIdx.x);
+  __syncthreads();
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < ncell;
+       base += stride) {
+    const long long g = base + (threadIdx.x & 31);
+    const bool valid = g < ncell;
+    const size_t c = valid ? (size_t)(g / nx) * P.pitch + (size_t)(g % nx) : 0;
+    bool newton = false, go_on = false, warm_cell = false;
+    int fin = 0;
+    unsigned tr = 0;
+    float fw[WARM_IN];
+    if (valid && mask[c]) {
+      double q0[NV], Xc[NV], qsi[NV], Rj[NV], bx, by;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        q0[i] = q[c + i * N];
+        Xc[i] = X[c + i * N];
+      }
+      newton = stage2_start<NS>(P, q0, Xc, c, Bx, By, Bxx, Bxy, Byy, gc, dt, qsi, Rj, bx, by);
+      W.status[c] = newton ? 1 : 0;
+      if (newton) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-          q0[i] = q[c + i * N];
-          Xc[i] = X[c + i * N];
+          W.qsi[c + i * N] = qsi[i];
+          W.Rj[c + i * N] = Rj[i];
         }
-        // q_fv = q0 - dt*(MATMUL(divFlux-expl, a_tilde) - MATMUL(NH+SI_NH, a_dirk))
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          double sa = (0.0 + Xc[i] * 1.0) + (0.0 - 0.0) * 0.0;
-          double sb = (0.0 + (0.0 + 0.0) * 0.0) + (0.0 + 0.0) * 0.0;
-          qfv[i] = q0[i] - dt * (sa - sb);
-        }
-        double qg[NV];
-        if (qfv[0] > 0.0) {
-          double qpv[NP];
-          qc_to_qp<NS>(P, qfv, qpv);
-          const double bx = Bx[c], by = By[c];
-          double bxx = 0.0, bxy = 0.0, byy = 0.0, gcf = 1.0;
-          if (P.curvature_term_flag) {
-            bxx = Bxx[c];
-            bxy = Bxy[c];
-            byy = Byy[c];
-          }
-          if (P.slope_correction_flag) gcf = gc[c];
-          double si2, si3;
-          semi_impl_terms<NS>(P, bx, by, bxx, bxy, byy, gcf, qpv, si2, si3);
-          double SI[NV], qsi[NV];
-#pragma unroll
-          for (int i = 0; i < NV; ++i) SI[i] = (i == 1) ? si2 : ((i == 2) ? si3 : 0.0);
-#pragma unroll
-          for (int i = 0; i < NV; ++i) qsi[i] = qfv[i] + dt * 1.0 * SI[i];
-          if (qfv[1] * qfv[1] + qfv[2] * qfv[2] == 0.0) {
-            qsi[1] = 0.0;
-            qsi[2] = 0.0;
-          } else if (qsi[1] * qfv[1] < 0.0 || qsi[2] * qfv[2] < 0.0) {
-            qsi[1] = 0.0;
-            qsi[2] = 0.0;
-          } else {
-            double Sm = sqrt(qsi[1] * qsi[1] + qsi[2] * qsi[2]);
-            double Fm = sqrt(qfv[1] * qfv[1] + qfv[2] * qfv[2]);
-            qsi[1] = Sm * qfv[1] / Fm;
-            qsi[2] = Sm * qfv[2] / Fm;
-          }
-          double Rj[NV];
-#pragma unroll
-          for (int i = 0; i < NV; ++i) {
-            // rows other than 2, 3: qsi = qfv + dt*0 (or +0 for qfv = -0), so
-            // for finite qfv and a finite dt > 0 the difference is +0 and so
-            // is the quotient
-            if (i != 1 && i != 2 && isfinite(qfv[i]) && dt > 0.0 && dt < 1e300) SI[i] = 0.0;
-            else SI[i] = (qsi[i] - qfv[i]) / (dt * 1.0);
-            double sa = 0.0 + Xc[i] * 1.0;
-            double sb = 0.0 + (0.0 + 0.0) * 0.0;
-            Rj[i] = (sa - sb) - 1.0 * SI[i];
-            qg[i] = qsi[i];
-            W.qsi[c + i * N] = qsi[i];
-            W.Rj[c + i * N] = Rj[i];
-          }
-          W.status[c] = 1;
-          cells += 1;
+      }
+      if (newton && W.warm) {
+        // Newton waits for the network's guess (k_warm_predict, k_stage2_wstart)
+        warm_features<NS>(qsi, q0, Rj, dt, bx, by, fw);
+        warm_cell = true;
+      } else {
+        if (newton) {
           double qj_org[NV], qj_rel[NV], rt[NV], scal_f;
-          if (W.warm) {
-            // Newton waits for the network's guess (k_warm_predict, k_stage2_wstart)
-            warm_features<NS>(qsi, q0, Rj, dt, bx, by, fw);
-            warm_cell = true;
-          } else {
-          newton_scale<NS>(qg, qj_org);
-          if (newton_start<NS>(P, qg, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f)) {
+          bool need_rt, stale = false;
+          if (newton_begin<NS, 1>(P, qsi, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f, need_rt) ||
+              newton_step<NS, 1>(P, true, need_rt, q0, Rj, qj_org, bx, by, dt, qj_rel, rt, scal_f,
+                                 tr, stale)) {
             fin = 1;
-          } else if (newton_iter1<NS>(P, qg, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f)) {
-            fin = 1;
+#pragma unroll
+            for (int i = 0; i < NV; ++i) qsi[i] = qj_rel[i] * qj_org[i];
           } else {
             go_on = true;
 #pragma unroll
@@ -2091,216 +2576,27 @@ __device__ __forceinline__ void stage2_first_lane(
               W.rt[c + i * N] = rt[i];
             }
             W.sf[c] = scal_f;
+            W.status[c] = (1 << 2) | 1;
           }
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < NV; ++i) qg[i] = qfv[i];
-          W.status[c] = 0;
         }
-        if (!go_on && !warm_cell) {
+        if (!go_on) {
 #pragma unroll
-          for (int i = 0; i < NV; ++i) W.x[c + i * N] = qg[i];
+          for (int i = 0; i < NV; ++i) W.x[c + i * N] = qsi[i];
         }
       }
     }
-  newton_finish_stats(clk, fin, it_sum, maxit);
-  list_append(go_on, (uint32_t)c, W.list[0], &clk->nw_count[0]);
-  if (W.warm) {
-    const unsigned int slot = list_append(warm_cell, (uint32_t)c, W.wlist, &clk->nw_count[3]);
-    if (warm_cell) {
+    stat_add(st, newton, fin, tr);
+    list_append(go_on, (uint32_t)c, W.list, &clk->nw_count[0]);
+    if (W.warm) {
+      const unsigned int slot = list_append(warm_cell, (uint32_t)c, W.wlist, &clk->nw_count[3]);
+      if (warm_cell) {
 #pragma unroll
-      for (int i = 0; i < WARM_IN; ++i) W.feat[(size_t)slot * WARM_IN + i] = fw[i];
+        for (int i = 0; i < WARM_IN; ++i) W.feat[(size_t)slot * WARM_IN + i] = fw[i];
+      }
     }
   }
-}
-
-// k_stage2_first: 80 registers (6 blocks of 128 per SM) measured faster
-// than 64 with its larger spill set.
-#ifndef IMEX_FIRST_MINB
-#define IMEX_FIRST_MINB 6
-#endif
-template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_FIRST_MINB)
-    k_stage2_first(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
-                   const double* __restrict__ X, const uint8_t* __restrict__ mask,
-                   const double* __restrict__ Bx, const double* __restrict__ By,
-                   const double* __restrict__ Bxx, const double* __restrict__ Bxy,
-                   const double* __restrict__ Byy, const double* __restrict__ gc, NewtonWork W,
-                   DevClock* clk) {
-  const DevParams& P = Pp;
-  const int nx = P.nx;
-  const long long ncell = (long long)nx * P.ny;
-  const double dt = clk->dt;
-  unsigned long long cells = 0, it_sum = 0, maxit = 0;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < ncell;
-       base += stride) {
-    const long long g = base + (threadIdx.x & 31);
-    const bool valid = g < ncell;
-    const size_t c = valid ? (size_t)(g / nx) * P.pitch + (size_t)(g % nx) : 0;
-    stage2_first_lane<NS>(P, q, X, mask, Bx, By, Bxx, Bxy, Byy, gc, W, clk, dt, valid, c, cells,
-                          it_sum, maxit);
-  }
-  newton_flush_stats(clk, cells, it_sum, 0, maxit);
-}
-
-// One Newton iteration (nl_iter = 2 or 3) for entry e of list nl_iter-2
-// (valid: e is inside the list); the lane takes part in the warp's list
-// appends whether or not it has a cell.
-template <int NS>
-__device__ __forceinline__ void stage2_iter_lane(const DevParams& P, const double* __restrict__ q,
-                                                 const double* __restrict__ Bx,
-                                                 const double* __restrict__ By, NewtonWork W,
-                                                 DevClock* clk, double dt, int nl_iter,
-                                                 bool valid, long long e,
-                                                 unsigned long long& it_sum,
-                                                 unsigned long long& maxit,
-                                                 unsigned long long& trials) {
-  constexpr int NV = 4 + NS;
-  const size_t N = (size_t)P.plane;
-  const uint32_t* in = W.list[nl_iter - 2];
-  uint32_t* out = W.list[nl_iter - 1];
-  {
-    uint32_t c = 0;
-    bool go_on = false, fb = false;
-    int fin = 0;
-    if (valid) {
-      c = in[e];
-      double q0[NV], Rj[NV], qj_org[NV], qj_rel[NV], rt[NV], qj[NV], scal_f;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        q0[i] = q[c + i * N];
-        Rj[i] = W.Rj[c + i * N];
-        qj[i] = W.qsi[c + i * N];
-        qj_rel[i] = W.x[c + i * N];
-        rt[i] = W.rt[c + i * N];
-      }
-      if (W.warm) {   // the Newton start (scaling source) was the network's guess
-        qj[1] = W.guess[c];
-        qj[2] = W.guess[c + N];
-      }
-      scal_f = W.sf[c];
-      bool stale = (W.status[c] & 2) != 0;
-      newton_scale<NS>(qj, qj_org);
-      long long tr = 0;
-      bool done = newton_iterk<NS>(P, qj, q0, Rj, Bx[c], By[c], dt, qj_org, qj_rel, rt, scal_f, tr,
-                                   stale);
-      trials += (unsigned long long)tr;
-      if (done || nl_iter >= NEWTON_MAX_IT) {
-        fin = nl_iter;
-        if (W.warm && (!done || !all_finite<NS>(qj))) {
-          fb = true;
-        } else {
-#pragma unroll
-          for (int i = 0; i < NV; ++i) W.x[c + i * N] = qj[i];
-        }
-      } else {
-        go_on = true;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          W.x[c + i * N] = qj_rel[i];
-          W.rt[c + i * N] = rt[i];
-        }
-        W.sf[c] = scal_f;
-        W.status[c] = stale ? 3 : 1;
-      }
-    }
-    newton_finish_stats(clk, fin, it_sum, maxit);
-    list_append(go_on, c, out, &clk->nw_count[nl_iter - 1]);
-    if (W.warm) list_append(fb, c, W.flist, &clk->nw_fb);
-  }
-}
-
-template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
-    k_stage2_iter(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
-                  const double* __restrict__ Bx, const double* __restrict__ By, NewtonWork W,
-                  DevClock* clk, int nl_iter) {
-  const DevParams& P = Pp;
-  const double dt = clk->dt;
-  const long long n = (long long)clk->nw_count[nl_iter - 2];
-  unsigned long long it_sum = 0, maxit = 0, trials = 0;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n;
-       base += stride) {
-    const long long e = base + (threadIdx.x & 31);
-    stage2_iter_lane<NS>(P, q, Bx, By, W, clk, dt, nl_iter, e < n, e, it_sum, maxit, trials);
-  }
-  newton_flush_stats(clk, 0, it_sum, trials, maxit);
-}
-
-// Iterations 4..100 for entry e of list 2.
-template <int NS>
-__device__ __forceinline__ void stage2_tail_lane(const DevParams& P, const double* __restrict__ q,
-                                                 const double* __restrict__ Bx,
-                                                 const double* __restrict__ By, NewtonWork W,
-                                                 DevClock* clk, double dt, bool valid,
-                                                 long long e, unsigned long long& it_sum,
-                                                 unsigned long long& maxit,
-                                                 unsigned long long& trials) {
-  constexpr int NV = 4 + NS;
-  const size_t N = (size_t)P.plane;
-  {
-    int fin = 0;
-    bool fb = false;
-    uint32_t c = 0;
-    if (valid) {
-      c = W.list[2][e];
-      double q0[NV], Rj[NV], qj_org[NV], qj_rel[NV], rt[NV], qj[NV], scal_f;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        q0[i] = q[c + i * N];
-        Rj[i] = W.Rj[c + i * N];
-        qj[i] = W.qsi[c + i * N];
-        qj_rel[i] = W.x[c + i * N];
-        rt[i] = W.rt[c + i * N];
-      }
-      if (W.warm) {
-        qj[1] = W.guess[c];
-        qj[2] = W.guess[c + N];
-      }
-      scal_f = W.sf[c];
-      bool stale = (W.status[c] & 2) != 0;
-      newton_scale<NS>(qj, qj_org);
-      const double bx = Bx[c], by = By[c];
-      int it;
-      for (it = 4; it <= NEWTON_MAX_IT; ++it) {
-        long long tr = 0;
-        bool done = newton_iterk<NS>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f, tr,
-                                     stale);
-        trials += (unsigned long long)tr;
-        if (done) break;
-      }
-      fin = it > NEWTON_MAX_IT ? NEWTON_MAX_IT : it;
-      if (W.warm && (it > NEWTON_MAX_IT || !all_finite<NS>(qj))) {
-        fb = true;
-      } else {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) W.x[c + i * N] = qj[i];
-      }
-    }
-    newton_finish_stats(clk, fin, it_sum, maxit);
-    if (W.warm) list_append(fb, c, W.flist, &clk->nw_fb);
-  }
-}
-
-template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
-    k_stage2_tail(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
-                  const double* __restrict__ Bx, const double* __restrict__ By, NewtonWork W,
-                  DevClock* clk) {
-  const DevParams& P = Pp;
-  const double dt = clk->dt;
-  const long long n = (long long)clk->nw_count[2];
-  unsigned long long it_sum = 0, maxit = 0, trials = 0;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n;
-       base += stride) {
-    const long long e = base + (threadIdx.x & 31);
-    stage2_tail_lane<NS>(P, q, Bx, By, W, clk, dt, e < n, e, it_sum, maxit, trials);
-  }
-  newton_flush_stats(clk, 0, it_sum, trials, maxit);
+  __syncthreads();
+  stat_flush(st, clk, threadIdx.x);
 }
 
 // The network's momentum guesses for the cells of the warm-start list:
@@ -2346,19 +2642,21 @@ __global__ void __launch_bounds__(32 * mlp::WARPS)
 }
 
 // Newton scaling and iteration 1 from the network's guess for the cells of
-// the warm-start list; cells still iterating go to list 0 as in
+// the warm-start list; cells still iterating go to the list as in
 // k_stage2_first.
 template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
+__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
     k_stage2_wstart(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
-                    const double* __restrict__ Bx, const double* __restrict__ By, NewtonWork W,
-                    DevClock* clk) {
+                    const double* __restrict__ Bx, const double* __restrict__ By,
+                    const __grid_constant__ NewtonWork W, DevClock* clk) {
   const DevParams& P = Pp;
   constexpr int NV = 4 + NS;
+  __shared__ NewtonStats st;
   const size_t N = (size_t)P.plane;
   const double dt = clk->dt;
   const long long n = (long long)clk->nw_count[3];
-  unsigned long long it_sum = 0, maxit = 0, trials = 0;
+  stat_reset(st, threadIdx.x);
+  __syncthreads();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n;
        base += stride) {
@@ -2366,6 +2664,7 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
     uint32_t c = 0;
     bool go_on = false, fb = false;
     int fin = 0;
+    unsigned tr = 0;
     if (e < n) {
       c = W.wlist[e];
       double q0[NV], Rj[NV], qj[NV], qj_org[NV], qj_rel[NV], rt[NV], scal_f;
@@ -2378,11 +2677,15 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
       qj[1] = W.guess[c];
       qj[2] = W.guess[c + N];
       const double bx = Bx[c], by = By[c];
-      newton_scale<NS>(qj, qj_org);
-      bool done = newton_start<NS>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f) ||
-                  newton_iter1<NS>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f);
+      bool need_rt, stale = false;
+      const bool done =
+          newton_begin<NS, 1>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f, need_rt) ||
+          newton_step<NS, 1>(P, true, need_rt, q0, Rj, qj_org, bx, by, dt, qj_rel, rt, scal_f, tr,
+                             stale);
       if (done) {
         fin = 1;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
         if (!all_finite<NS>(qj)) {
           fb = true;
         } else {
@@ -2397,21 +2700,23 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
           W.rt[c + i * N] = rt[i];
         }
         W.sf[c] = scal_f;
+        W.status[c] = (1 << 2) | 1;
       }
     }
-    newton_finish_stats(clk, fin, it_sum, maxit);
-    list_append(go_on, c, W.list[0], &clk->nw_count[0]);
+    stat_add(st, false, fin, tr);
+    list_append(go_on, c, W.list, &clk->nw_count[0]);
     list_append(fb, c, W.flist, &clk->nw_fb);
   }
-  newton_flush_stats(clk, 0, it_sum, trials, maxit);
+  __syncthreads();
+  stat_flush(st, clk, threadIdx.x);
 }
 
 // Warm starts that failed, redone with the plain start (q_si).
 template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_STAGE2_MINB)
+__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
     k_stage2_fallback(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
                       const double* __restrict__ Bx, const double* __restrict__ By,
-                      NewtonWork W, DevClock* clk) {
+                      const __grid_constant__ NewtonWork W, DevClock* clk) {
   const DevParams& P = Pp;
   constexpr int NV = 4 + NS;
   const size_t N = (size_t)P.plane;
@@ -2496,120 +2801,31 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// Sign guard after Newton (src/solver_2d.f90:1238-1255) and assemble_sol
-// (src/solver_2d.f90:1339-1626).
-template <int NS>
-__device__ __forceinline__ void stage2_post_cell(const DevParams& P, double* __restrict__ q,
-                                                 const uint8_t* __restrict__ cellinfo,
-                                                 NewtonWork W, DevClock* clk, int j, int k) {
-  constexpr int NV = 4 + NS, NP = 6 + NS;
-  const int nx = P.nx, ny = P.ny;
-  const size_t N = (size_t)P.plane;
-  const size_t c = (size_t)k * P.pitch + j;
-  {
-    double qc[NV];
-#pragma unroll
-    for (int i = 0; i < NV; ++i) qc[i] = W.x[c + i * N];
-    if (W.status[c] & 1) {
-      const double qs1 = W.qsi[c + N], qs2 = W.qsi[c + 2 * N];
-      if (ny == 1) qc[2] = 0.0;
-      if (nx == 1) qc[1] = 0.0;
-      if (qs1 * qs1 + qs2 * qs2 == 0.0) {
-        qc[1] = 0.0;
-        qc[2] = 0.0;
-      } else if (qc[1] * qs1 <= 0.0 && qc[2] * qs2 <= 0.0) {
-        qc[1] = 0.0;
-        qc[2] = 0.0;
-      } else {
-        double Sm = sqrt(qc[1] * qc[1] + qc[2] * qc[2]);
-        double Fm = sqrt(qs1 * qs1 + qs2 * qs2);
-        qc[1] = Sm * qs1 / Fm;
-        qc[2] = Sm * qs2 / Fm;
-      }
-    }
-    const long long cell = (long long)k * nx + j;
-    bool anynan = false;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) anynan |= isnan(qc[i]);
-    if (anynan) record_error(clk, 1, cell);
-    if (qc[0] < EPS) {
-      if (qc[0] > -1.0e-7) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) qc[i] = 0.0;
-      } else {
-        record_error(clk, 2, cell);
-      }
-    }
-    bool anyneg = false, anybad = false;
-#pragma unroll
-    for (int i = 0; i < NS; ++i) anyneg |= (qc[4 + i] < 0.0);
-    if (anyneg) {
-#pragma unroll
-      for (int i = 0; i < NS; ++i) anybad |= (qc[4 + i] <= -1.0e-7);
-      if (anybad) {
-        record_error(clk, 3, cell);
-      } else {
-#pragma unroll
-        for (int i = 0; i < NS; ++i)
-          if (qc[4 + i] > -1.0e-7) qc[4 + i] = 0.0;
-      }
-    }
-    double qpv[NP];
-    qc_to_qp<NS>(P, qc, qpv);
-    if (qpv[3] < 273.0) record_error(clk, 4, cell);
-    double ssum = 0.0;
-#pragma unroll
-    for (int i = 0; i < NS; ++i) ssum += qc[4 + i];
-    if (ssum > qc[0]) {
-      if ((ssum - qc[0]) / qc[0] < 1.0e-10 || qc[0] < EPS) {
-        double s = 0.0;
-#pragma unroll
-        for (int i = 0; i < NS; ++i) s += qc[4 + i];
-#pragma unroll
-        for (int i = 0; i < NS; ++i) qc[4 + i] = qc[4 + i] / s * qc[0];
-      } else {
-        record_error(clk, 5, cell);
-      }
-    }
-    if (P.has_cellinfo && (cellinfo[cell] & CI_NODATA)) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) qc[i] = 0.0;
-    }
-#pragma unroll
-    for (int i = 0; i < NV; ++i) q[c + i * N] = qc[i];
-  }
-}
-
+// Sign guard and assembly from the NewtonWork planes (learned start, harvest).
 template <int NS>
 __global__ void __launch_bounds__(STAGE2_THREADS)
     k_stage2_post(const __grid_constant__ DevParams Pp, double* __restrict__ q,
                   const uint8_t* __restrict__ mask, const uint8_t* __restrict__ cellinfo,
-                  NewtonWork W, DevClock* clk) {
+                  const __grid_constant__ NewtonWork W, DevClock* clk) {
   const DevParams& P = Pp;
+  constexpr int NV = 4 + NS;
   const int nx = P.nx;
+  const size_t N = (size_t)P.plane;
   const long long ncell = (long long)nx * P.ny;
   for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < ncell;
        g += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(g % nx), k = (int)(g / nx);
-    if (!mask[(size_t)k * P.pitch + j]) continue;
-    stage2_post_cell<NS>(P, q, cellinfo, W, clk, j, k);
-  }
-}
-
-// k_stage2_post over the grid rows [k0, k1) (imex_gpu_advance_host).
-template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS)
-    k_stage2_post_rows(const __grid_constant__ DevParams Pp, double* __restrict__ q,
-                       const uint8_t* __restrict__ mask, const uint8_t* __restrict__ cellinfo,
-                       NewtonWork W, DevClock* clk, int k0, int k1) {
-  const DevParams& P = Pp;
-  const int nx = P.nx;
-  const long long ncell = (long long)nx * (k1 - k0);
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < ncell;
-       g += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(g % nx), k = k0 + (int)(g / nx);
-    if (!mask[(size_t)k * P.pitch + j]) continue;
-    stage2_post_cell<NS>(P, q, cellinfo, W, clk, j, k);
+    const size_t c = (size_t)k * P.pitch + j;
+    if (!mask[c]) continue;
+    double qc[NV], qs1 = 0.0, qs2 = 0.0;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) qc[i] = W.x[c + i * N];
+    const bool newton = (W.status[c] & 1) != 0;
+    if (newton) {
+      qs1 = W.qsi[c + N];
+      qs2 = W.qsi[c + 2 * N];
+    }
+    stage2_assemble<NS>(P, qc, newton, qs1, qs2, q, cellinfo, clk, j, k);
   }
 }
 

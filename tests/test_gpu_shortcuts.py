@@ -85,3 +85,55 @@ def test_flux_edges_bitexact(kind):
         o.post_step()
         np.testing.assert_array_equal(o.get_state(), g.get_state(), err_msg="%s step %d" % (kind, step))
         t += dto
+
+
+@pytest.mark.parametrize("rheology", [1, 6])
+@pytest.mark.parametrize("kind", ["still", "creeping", "small_loads", "ambient", "no_energy", "tilted"])
+def test_newton_edges_bitexact(kind, rheology):
+    """States at and beyond the edges of the Newton solve's shared
+    evaluation: cells at rest, speeds whose squares underflow, components below the
+    scaling floor of 1e-3 (where (q/q_org)*q_org need not be q), densities next to
+    the ambient one, no kinetic energy in T, slope correction."""
+    import cases
+    from imex_sflow2d_v2_b200 import configs
+    from imex_sflow2d_v2_b200.solver import ImexSolver
+    from oracle import Oracle
+    p, st, q = cases.sloped(n=40, rheology=rheology) if kind == "tilted" else \
+        cases.dambreak_ns(3, nx=40, ny=21, rheology=rheology)
+    q = np.array(q)
+    rng = np.random.default_rng(5)
+    shape = q[0].shape
+    wet = q[0] > 0.0
+    if kind == "still":
+        q[1:3] = 0.0
+        q[1, ::3] = 1e-9
+    elif kind == "creeping":
+        q[1] = np.where(wet, 10.0 ** rng.uniform(-200, -3, shape), 0.0)
+        q[2] = np.where(wet, -10.0 ** rng.uniform(-200, -3, shape), 0.0)
+    elif kind == "small_loads":
+        f = 10.0 ** rng.uniform(-9, 0, shape)
+        q = q * f
+        q[1], q[2] = q[0] * rng.normal(0.0, 2.0, shape), q[0] * rng.normal(0.0, 2.0, shape)
+    elif kind == "ambient":
+        q[4:] *= 10.0 ** rng.uniform(-14, 0, shape)
+        q[1] = q[0] * rng.normal(0.0, 1.0, shape)
+    elif kind == "no_energy":
+        p.energy_flag = 0
+        q[1] = q[0] * rng.normal(0.0, 5.0, shape)
+    o, g = Oracle(p, st, threads=4), ImexSolver(p, st)
+    for s in (o, g):
+        s.set_state(q, 0.0)
+    t = 0.0
+    for step in range(5):
+        o.check_solve(t)
+        g.check_solve(t)
+        dt = o.timestep()
+        assert dt == g.timestep()
+        o.rk_step(t, dt)
+        g.imex_RK_solver(t, dt)
+        o.post_step()
+        so, sg = o.stats(), g.stats()
+        np.testing.assert_array_equal(o.get_state(), g.get_state(), err_msg="%s step %d" % (kind, step))
+        assert (so.newton_cells, so.newton_iters, so.lnsrch_trials, list(so.newton_hist)) == \
+            (sg.newton_cells, sg.newton_iters, sg.lnsrch_trials, list(sg.newton_hist))
+        t += dt

@@ -90,21 +90,18 @@ def workload(n, layer):
     return configs.fractal_inlet(n=n, initial_layer=layer)
 
 
-def bytes_per_cell(ns, erosion, listed=(1.0, 0.0, 0.0)):
+def bytes_per_cell(ns, erosion):
     """Algorithmic bytes per grid cell and step of each timed kernel group
-    (8-byte values, 1-byte masks, 4-byte list entries).  `listed` is the
-    fraction of cells that run Newton iteration 2, 3 and 4.. (each such pass
-    reads and writes the cell's Newton state)."""
+    (8-byte values, 1-byte masks).  stage2_first is the whole of stage 2;
+    stage2_iter, the list of the few cells it leaves, and stage2_post, which runs
+    with the learned start only, add none."""
     nv = 4 + ns
     out = {
         "mask": 8 + 1,                                  # q1 read, mask byte written
         "flux": 8 * nv + 1 + 16 + 8 * nv,               # q, mask, B'x, B'y read; X written
-        # q, X, mask, B' read; q_si, Rj, iterate, residual, |r|^2, status, list written
-        "stage2_first": 16 * nv + 17 + 32 * nv + 8 + 1 + 4,
-        # per pass and listed cell: q, Rj, q_si, iterate, residual, |r|^2, B', list
-        # read; iterate, residual, |r|^2, list written
-        "stage2_iter": sum(listed) * (40 * nv + 8 + 16 + 4 + 16 * nv + 8 + 4),
-        "stage2_post": 8 * nv + 1 + 16 + 1 + 8 * nv,    # iterate, status, q_si(2), mask; q
+        "stage2_first": 16 * nv + 1 + 16 + 8 * nv,      # q, X, mask, B' read; q written
+        "stage2_iter": 0,
+        "stage2_post": 0,
     }
     if erosion:                                         # q, mask, B' read; q written;
         out["erosion"] = 8 * nv + 1 + 16 + 8 * nv + 2 * 3 * 8 * ns  # 3 planes per class r+w
@@ -747,8 +744,7 @@ def main():
     erosion = bool(p.erosion_coeff != 0.0 or p.settling_flag)
     hist = list(s1.newton_hist)
     ncells_newton = max(1, s1.newton_cells)
-    listed = (sum(hist[1:]) / cells, sum(hist[2:]) / cells, sum(hist[3:]) / cells)
-    bpc = bytes_per_cell(p.n_solid, erosion, listed)
+    bpc = bytes_per_cell(p.n_solid, erosion)
     timed = {k: v for k, v in kt.items() if v[1] > 0}
     dom = max(timed, key=lambda k: timed[k][0])
     steps_timed = args.steps

@@ -270,10 +270,11 @@ int imex_gpu_device_state(ImexCtx* ctx, double** q_dev, int64_t* pitch);
  * imex_gpu_advance launches without a graph, on the context stream;
  * imex_gpu_kernel_times returns, per kernel id, the summed event time in ms
  * and the number of timed launches since the last call.  Ids: 0 mask,
- * 1 flux (stage 1 + CFL), 2 stage 2 up to Newton iteration 1, 3 Newton
- * iterations 2.. (three launches), 4 stage-2 assembly, 5 erosion/deposition;
- * n_kernels must be at least 6.  imex_gpu_measure_fp64_peak times an FP64 FMA-chain kernel
- * and returns the achieved GFLOP/s (2 flops per FMA). */
+ * 1 flux (stage 1 + CFL), 2 stage 2, 3 its remaining cells (the list of large
+ * steps; with the learned start or the harvest, which keep stage 2 in passes, 2 is the
+ * start and 3 the Newton iterations), 4 stage-2 assembly (those passes only),
+ * 5 erosion/deposition; n_kernels must be at least 6.  imex_gpu_measure_fp64_peak times
+ * an FP64 FMA-chain kernel and returns the achieved GFLOP/s (2 flops per FMA). */
 int imex_gpu_profile(ImexCtx* ctx, int enable);
 int imex_gpu_kernel_times(ImexCtx* ctx, double* total_ms, int64_t* launches, int n_kernels);
 int imex_gpu_measure_fp64_peak(int device, double* gflops);
@@ -370,8 +371,9 @@ int imex_gpu_harvest_data(ImexCtx* ctx, const float** x_dev, const float** y_dev
  * batched instead: every phase of the step is one persistent kernel for all
  * members (a fixed grid walking device-built work lists: all tiles for the
  * mask, the tiles holding a solve cell for the fluxes, stage 2 and erosion,
- * the members' Newton lists laid end to end for the iteration passes), 13
- * or 14 launches per step for the whole ensemble, captured once in a CUDA
+ * the members' lists of remaining stage-2 cells laid end to end), 6 or 7
+ * launches per step for the whole ensemble, and 3 more when the members'
+ * tiles hold 262144 cells or more, captured once in a CUDA
  * graph and replayed.  Its first six steps are timed with the tile shapes
  * of the mask and flux passes (32x8, 16x16, 32x4 cells) in the order
  * 1 2 3 3 2 1, and the shape with the smallest total is kept;

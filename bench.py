@@ -92,19 +92,31 @@ def workload(n, layer):
 
 def bytes_per_cell(ns, erosion):
     """Algorithmic bytes per grid cell and step of each timed kernel group
-    (8-byte values, 1-byte masks).  stage2_first is the whole of stage 2;
-    stage2_iter, the list of the few cells it leaves, and stage2_post, which runs
-    with the learned start only, add none."""
+    (8-byte values, 1-byte masks).  Stage 2 is one group (roofline_groups): its
+    algorithm reads and writes a cell once, whether or not the cell goes on
+    through the list."""
     nv = 4 + ns
     out = {
         "mask": 8 + 1,                                  # q1 read, mask byte written
         "flux": 8 * nv + 1 + 16 + 8 * nv,               # q, mask, B'x, B'y read; X written
-        "stage2_first": 16 * nv + 1 + 16 + 8 * nv,      # q, X, mask, B' read; q written
-        "stage2_iter": 0,
-        "stage2_post": 0,
+        "stage2": 16 * nv + 1 + 16 + 8 * nv,            # q, X, mask, B' read; q written
     }
     if erosion:                                         # q, mask, B' read; q written;
         out["erosion"] = 8 * nv + 1 + 16 + 8 * nv + 2 * 3 * 8 * ns  # 3 planes per class r+w
+    return out
+
+
+STAGE2_PARTS = ("stage2_first", "stage2_iter", "stage2_post")
+
+
+def roofline_groups(values):
+    """A {timed kernel: number} record (times, counts, bytes) with the parts of
+    stage 2 added up: its list (stage2_iter) takes cells over from the main
+    kernel, so only the sum stands for a cell's work."""
+    out = {k: v for k, v in values.items() if k not in STAGE2_PARTS}
+    parts = [values[k] for k in STAGE2_PARTS if values.get(k)]
+    if parts:
+        out["stage2"] = sum(parts)
     return out
 
 
@@ -663,7 +675,7 @@ def roofline_line(dom, fp64, achieved, peak, peak_src, traffic, alg_bytes, avg_s
     launch, whose ratio to `alg_bytes_per_launch` measures re-reads and
     spills) and `hbm_frac_s8d` (the whole step against the fused minimum of
     `s8d_bytes_per_cell`)."""
-    fp64_bound = fp64 is not None and dom in ("flux", "stage2_first", "stage2_iter", "erosion")
+    fp64_bound = fp64 is not None and dom in ("flux", "stage2", "erosion")
     line = {"kernel": dom,
             "bound": "fp64" if fp64_bound else "hbm",
             "achieved": fp64["achieved_inst_per_s"] / 1e12 if fp64_bound else achieved,
@@ -746,9 +758,10 @@ def main():
     ncells_newton = max(1, s1.newton_cells)
     bpc = bytes_per_cell(p.n_solid, erosion)
     timed = {k: v for k, v in kt.items() if v[1] > 0}
-    dom = max(timed, key=lambda k: timed[k][0])
+    group_ms = roofline_groups({k: v[0] for k, v in timed.items()})
+    dom = max(group_ms, key=group_ms.get)
     steps_timed = args.steps
-    dom_ms = timed[dom][0] / steps_timed            # per step (a group may be several launches)
+    dom_ms = group_ms[dom] / steps_timed            # per step (a group may be several launches)
     avg_s = dom_ms * 1e-3
     alg_bytes = bpc[dom] * cells
     peak = None
@@ -762,7 +775,7 @@ def main():
     traffic = None
     try:
         tr = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))
-        traffic = tr.get(dom)
+        traffic = roofline_groups(tr).get(dom)
     except Exception:
         pass
     fp64_peak = None
@@ -772,12 +785,12 @@ def main():
         pass
     # FP64 pipe: instructions per cell (ncu) x cells / live kernel time, against
     # the measured FMA-chain peak (one FP64 instruction per lane per FMA)
-    fpc = fp64_counts().get(BUILD_MODE, {})
+    fpc = roofline_groups(fp64_counts().get(BUILD_MODE, {}))
     fp64 = None
     fp64_all = {}
     if fp64_peak:
         peak_inst_s = fp64_peak * 1e9 / 2.0
-        for k_, (tot_ms, _) in timed.items():
+        for k_, tot_ms in group_ms.items():
             if fpc.get(k_):
                 fp64_all[k_] = fpc[k_] * cells / (tot_ms / steps_timed * 1e-3) / peak_inst_s
         if dom in fpc:

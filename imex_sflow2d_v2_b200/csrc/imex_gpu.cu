@@ -354,8 +354,8 @@ cudaError_t launch_stage2_ns(ImexCtx* ctx) {
     }
   }
   if (ctx->nw.harvest) {
-    k_harvest<NS><<<grid_1d(ncell, 128), 128, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx, ctx->By,
-                                                                ctx->nw, ctx->clk);
+    k_harvest<NS><<<grid_1d(ncell, 128), 128, 0, ctx->stream>>>(
+        ctx->P, ctx->q, ctx->mask, ctx->Bx, ctx->By, ctx->nw, ctx->clk);
     ctx->launches += 1;
   }
   {

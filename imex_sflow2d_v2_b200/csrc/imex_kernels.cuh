@@ -2750,12 +2750,14 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
 // Training pairs from the finished Newton solves (before the sign guard):
 // the inputs of warm_features and the momentum change per unit q(1), for
 // every hstride-th Newton cell (cells taken by a hash of their index and
-// the step, so that successive steps sample different cells).
+// the step, so that successive steps sample different cells).  Only cells of the
+// present mask: this step has written the planes of no others, where an earlier
+// step may have left a solve, or (k_stage2's list) the middle of one.
 template <int NS>
 __global__ void __launch_bounds__(128)
     k_harvest(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
-              const double* __restrict__ Bx, const double* __restrict__ By, NewtonWork W,
-              DevClock* clk) {
+              const uint8_t* __restrict__ mask, const double* __restrict__ Bx,
+              const double* __restrict__ By, NewtonWork W, DevClock* clk) {
   const DevParams& P = Pp;
   constexpr int NV = 4 + NS;
   const int nx = P.nx;
@@ -2773,7 +2775,7 @@ __global__ void __launch_bounds__(128)
       c = (size_t)(g / nx) * P.pitch + (size_t)(g % nx);
       unsigned long long h = ((unsigned long long)g + salt) * 0xBF58476D1CE4E5B9ULL;
       h ^= h >> 31;
-      if ((W.status[c] & 1) && (h % W.hstride) == 0) {
+      if (mask[c] && (W.status[c] & 1) && (h % W.hstride) == 0) {
         double q0[NV], qsi[NV], Rj[NV], x1, x2;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {

@@ -66,7 +66,7 @@ struct ImexCtx {
   uint32_t* post_vuln = nullptr;
   double* post_diag = nullptr;
   double* nw_buf = nullptr;      // backing store of nw's FP64 planes
-  uint32_t* nw_lists = nullptr;  // backing store of nw's cell list
+  uint32_t* nw_lists = nullptr;  // backing store of nw's cell lists
   // learned warm start and training-pair harvest
   struct ImexMLP* warm_mlp = nullptr;  // not owned
   uint32_t* nw_wlist = nullptr;
@@ -147,6 +147,8 @@ cudaError_t upload_plane(ImexCtx* ctx, double* dst, const double* src, double fi
     for (int k = 0; k < ny; ++k) std::memcpy(&h[(size_t)k * pitch], src + (size_t)k * nx, nx * sizeof(double));
   return cudaMemcpy(dst, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
 }
+
+unsigned long long grid_cells(const DevParams& P) { return (unsigned long long)P.nx * P.ny; }
 
 dim3 tile_grid(const DevParams& P) { return dim3((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY); }
 
@@ -276,7 +278,7 @@ cudaError_t launch_flux(ImexCtx* ctx) {
 cudaError_t launch_warm_predict(ImexCtx* ctx);  // after ImexMLP (below)
 
 template <int NS, int T, bool LIST>
-cudaError_t launch_stage2_blocks(ImexCtx* ctx, int k0, int k1, unsigned long long list_min) {
+cudaError_t launch_stage2_blocks(ImexCtx* ctx, int k0, int k1, bool list_form) {
   const size_t smem = sizeof(NewtonShared<NS, T>);
   static std::atomic<unsigned long long> attr{0};
   if (attr_needed(attr)) {
@@ -287,7 +289,7 @@ cudaError_t launch_stage2_blocks(ImexCtx* ctx, int k0, int k1, unsigned long lon
   }
   k_stage2<NS, T, LIST><<<grid_1d((long long)ctx->P.nx * (k1 - k0), T), T, smem, ctx->stream>>>(
       ctx->P, ctx->q, ctx->X, ctx->mask, ctx->cellinfo, ctx->Bx, ctx->By, ctx->Bxx, ctx->Bxy,
-      ctx->Byy, ctx->gc, ctx->nw, ctx->clk, k0, k1, list_min);
+      ctx->Byy, ctx->gc, ctx->nw, ctx->clk, k0, k1, list_form);
   ctx->launches += 1;
   return cudaGetLastError();
 }
@@ -301,15 +303,15 @@ cudaError_t launch_stage2_rows(ImexCtx* ctx, int k0, int k1) {
   cudaError_t e;
   if ((long long)P.nx * P.ny < (long long)LIST_MIN_CELLS) {
     ProfScope ps(ctx, KID_S2_FIRST);
-    return launch_stage2_blocks<NS, STAGE2_THREADS, false>(ctx, k0, k1, ~0ULL);
+    return launch_stage2_blocks<NS, STAGE2_THREADS, false>(ctx, k0, k1, false);
   }
-  k_nw_reset<<<1, 1, 0, ctx->stream>>>(ctx->clk);
+  k_stage2_form<<<1, 1, 0, ctx->stream>>>(ctx->P, ctx->nw, ctx->clk);
   ctx->launches += 1;
   {
     ProfScope ps(ctx, KID_S2_FIRST);
-    e = launch_stage2_blocks<NS, 512, true>(ctx, k0, k1, LIST_MIN_CELLS);
+    e = launch_stage2_blocks<NS, 512, true>(ctx, k0, k1, true);
     if (e == cudaSuccess)
-      e = launch_stage2_blocks<NS, STAGE2_THREADS, false>(ctx, k0, k1, LIST_MIN_CELLS);
+      e = launch_stage2_blocks<NS, STAGE2_THREADS, false>(ctx, k0, k1, true);
     if (e != cudaSuccess) return e;
   }
   ProfScope ps(ctx, KID_S2_ITER);
@@ -444,7 +446,8 @@ cudaError_t launch_post_diag(ImexCtx* ctx) {
 cudaError_t launch_mask(ImexCtx* ctx, int solve_all = 0) {
   const DevParams& P = ctx->P;
   k_mask<<<tile_grid(P), 256, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->release, ctx->cellinfo,
-                                                ctx->clk, ctx->mask, ctx->clk, solve_all);
+                                                ctx->clk, ctx->mask, ctx->clk, solve_all,
+                                                solve_all ? nullptr : ctx->nw.cells);
   ctx->launches += 1;
   return cudaGetLastError();
 }
@@ -458,7 +461,7 @@ bool erosion_active(const ImexCtx* ctx) {
 // , erosion/deposition, t += dt.
 cudaError_t enqueue_step(ImexCtx* ctx) {
   cudaError_t e;
-  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 1);
+  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 1, grid_cells(ctx->P));
   ctx->launches += 1;
   {
     ProfScope ps(ctx, KID_MASK);
@@ -523,7 +526,7 @@ cudaError_t enqueue_host_step_ns(ImexCtx* ctx, const double* q_in, double* q_out
       return e;
     if ((e = cudaEventRecord(ev[1 + b], cs)) != cudaSuccess) return e;
   }
-  k_step_begin<<<1, 1, 0, st>>>(ctx->clk, P.max_dt, 1);
+  k_step_begin<<<1, 1, 0, st>>>(ctx->clk, P.max_dt, 1, grid_cells(P));
   const size_t smem = sizeof(FluxShared<NS>);
   static std::atomic<unsigned long long> attr_set{0};
   if (attr_needed(attr_set)) {
@@ -952,13 +955,14 @@ int imex_gpu_create(const ImexParams* p, const ImexStatic* s, int device, ImexCt
   // stage-2 Newton state: q_si, Rj, iterate, residual (nv planes each), |r|^2/2
   CK(dalloc(&ctx->nw_buf, plane * (4 * (size_t)nv + 1)));
   CK(dalloc(&ctx->nw.status, plane));
-  CK(dalloc(&ctx->nw_lists, plane));
+  CK(dalloc(&ctx->nw_lists, plane * 2));
   ctx->nw.qsi = ctx->nw_buf;
   ctx->nw.Rj = ctx->nw_buf + plane * nv;
   ctx->nw.x = ctx->nw_buf + plane * nv * 2;
   ctx->nw.rt = ctx->nw_buf + plane * nv * 3;
   ctx->nw.sf = ctx->nw_buf + plane * nv * 4;
   ctx->nw.list = ctx->nw_lists;
+  if (grid_cells(P) >= DENSE_MIN_GRID) ctx->nw.cells = ctx->nw_lists + plane;
   CK(cudaDeviceSynchronize());
   *out = ctx;
   return IMEX_OK;
@@ -1076,8 +1080,9 @@ int imex_gpu_check_solve(ImexCtx* ctx, double t, int solve_all, int64_t* n_solve
   CK(cudaSetDevice(ctx->device));
   int r = push_time(ctx, t, nullptr);
   if (r) return r;
-  const unsigned long long zero = 0;
-  CK(cudaMemcpyAsync(&ctx->clk->solve_cells, &zero, sizeof(unsigned long long), cudaMemcpyHostToDevice, ctx->stream));
+  static_assert(offsetof(DevClock, n_listed) == offsetof(DevClock, solve_cells) + 8, "reset as one");
+  const unsigned long long zero[2] = {0, 0};
+  CK(cudaMemcpyAsync(&ctx->clk->solve_cells, zero, sizeof(zero), cudaMemcpyHostToDevice, ctx->stream));
   CK(launch_mask(ctx, solve_all ? 1 : 0));
   ctx->x_valid = false;
   unsigned long long cnt = 0;
@@ -1090,7 +1095,7 @@ int imex_gpu_check_solve(ImexCtx* ctx, double t, int solve_all, int64_t* n_solve
 int imex_gpu_timestep(ImexCtx* ctx, double* dt) {
   if (!ctx || !dt) return IMEX_EINVAL;
   CK(cudaSetDevice(ctx->device));
-  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 0);
+  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 0, grid_cells(ctx->P));
   ctx->launches += 1;
   if (ctx->P.cfl != -1.0) {
     CK(launch_flux(ctx));

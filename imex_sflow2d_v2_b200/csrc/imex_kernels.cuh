@@ -70,13 +70,15 @@ struct DevClock {
   unsigned long long newton_cells, newton_iters, lnsrch_trials, newton_maxit;
   unsigned long long hist[16];
   unsigned long long solve_cells;
+  unsigned long long n_listed;       // solve cells written to NewtonWork's `cells`, or
+                                     // 2^62: not listed in this step
   unsigned long long steps;
   unsigned int nw_count[4];  // cells appended to the stage-2 Newton lists
                              // ([3]: the warm-start list)
   unsigned long long harvest_n;      // training pairs written so far
   unsigned long long warm_fallback;  // warm starts redone from q_si
   unsigned int nw_fb;                // cells in the warm-start fallback list
-  int pad2_;
+  int use_list;                      // k_stage2's form in this step (k_stage2_form)
 };
 
 IMEX_HD double x_stag(const DevParams& P, int J) { return P.x0 + (double)(J - 1) * P.dx; }
@@ -105,16 +107,23 @@ __device__ const RingCell* find_ring(const RingCell* ring, int n, long long idx)
 // check_solve(.FALSE.) for n_RK = 2 on the tile whose first cell is
 // (j0, k0): the wet/source seed of the tile and a 2-cell halo, two 4-point
 // dilations, the border rows and the inlet-interior removal.  Returns, to
-// every thread of the block, whether any cell of the tile is solved.
+// every thread of the block, whether any cell of the tile is solved.  With `cells`
+// the solve cells are also appended there (a tile of one cell per thread), until
+// they are half the grid's: stage 2 takes the list of sparse steps only
+// (DENSE_MIN_GRID).
 template <class TS>
 __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __restrict__ q1,
                                           const double* __restrict__ release_time,
                                           const uint8_t* __restrict__ cellinfo, double t,
                                           uint8_t* __restrict__ mask, DevClock* clkw,
                                           int solve_all, int j0, int k0,
-                                          uint8_t (*s0)[TS::SW], uint8_t (*s1)[TS::SW]) {
+                                          uint8_t (*s0)[TS::SW], uint8_t (*s1)[TS::SW],
+                                          uint32_t* __restrict__ cells = nullptr) {
   constexpr int SWt = TS::SW, SHt = TS::SH, TXt = TS::TX, TYt = TS::TY;
   const int nx = P.nx, ny = P.ny;
+  __shared__ bool list;
+  unsigned long long listed = 0;   // loaded here, looked at behind the tile's loads
+  if (cells && threadIdx.x == 0) listed = *(volatile unsigned long long*)&clkw->n_listed;
   for (int e = threadIdx.x; e < SWt * SHt; e += blockDim.x) {
     int lx = e % SWt, ly = e / SWt;
     int j = j0 + lx - HALO, k = k0 + ly - HALO;
@@ -132,6 +141,7 @@ __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __re
     }
     s0[ly][lx] = m;
   }
+  if (threadIdx.x == 0) list = 2 * listed < (unsigned long long)nx * ny;
   __syncthreads();
   // first dilation on the tile plus a 1-cell ring
   for (int e = threadIdx.x; e < SWt * SHt; e += blockDim.x) {
@@ -145,6 +155,7 @@ __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __re
   }
   __syncthreads();
   int cnt = 0;
+  size_t cell = 0;
   for (int e = threadIdx.x; e < TXt * TYt; e += blockDim.x) {
     int lx = e % TXt + HALO, ly = e / TXt + HALO;
     int j = j0 + lx - HALO, k = k0 + ly - HALO;
@@ -153,9 +164,11 @@ __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __re
     if (j >= 1 && j < nx - 1 && k >= 1 && k < ny - 1)
       m = m | s1[ly][lx - 1] | s1[ly][lx + 1] | s1[ly - 1][lx] | s1[ly + 1][lx];
     if (P.radial_source_flag && (cellinfo[(size_t)k * nx + j] & CI_SRC_MASK) == 1) m = 0;
-    mask[(size_t)k * P.pitch + j] = m;
+    cell = (size_t)k * P.pitch + j;
+    mask[cell] = m;
     cnt += m;
   }
+  const bool solve = cnt != 0;
   // the block's solve cells, in one atomic add: those to one address are served
   // one by one, and an add per warp bound the kernel (0.099 ms on 2048^2 solve
   // cells, 0.065 now)
@@ -166,6 +179,16 @@ __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __re
   int total = 0;
   for (int w = 0; w < (int)(blockDim.x >> 5); ++w) total += warp_cnt[w];
   if (threadIdx.x == 0 && total) atomicAdd(&clkw->solve_cells, (unsigned long long)total);
+  if (cells && list && total) {
+    __shared__ unsigned first;
+    if (threadIdx.x == 0)
+      first = (unsigned)atomicAdd(&clkw->n_listed, (unsigned long long)total);
+    __syncthreads();
+    const unsigned m = __ballot_sync(0xffffffffu, solve);
+    unsigned slot = first + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) slot += warp_cnt[w];
+    if (solve) cells[slot] = (uint32_t)cell;
+  }
   return total != 0;
 }
 
@@ -173,11 +196,13 @@ __global__ void __launch_bounds__(256) k_mask(const __grid_constant__ DevParams 
                                               const double* __restrict__ release_time,
                                               const uint8_t* __restrict__ cellinfo,
                                               const DevClock* clk, uint8_t* __restrict__ mask,
-                                              DevClock* clkw, int solve_all) {
+                                              DevClock* clkw, int solve_all,
+                                              uint32_t* __restrict__ cells) {
+  static_assert(TX * TY == 256, "one cell per thread");
   __shared__ uint8_t s0[SH][SW];
   __shared__ uint8_t s1[SH][SW];
   mask_tile<Shape32x8>(Pp, q1, release_time, cellinfo, clk->t, mask, clkw, solve_all,
-                       blockIdx.x * TX, blockIdx.y * TY, s0, s1);
+                       blockIdx.x * TX, blockIdx.y * TY, s0, s1, cells);
 }
 
 // ------------------------------------------------------ TMA tile loads
@@ -1959,6 +1984,7 @@ struct NewtonWork {
                     // residual must be evaluated again (see newton_step); listed
                     // cells: iterations taken in the upper bits
   uint32_t* list;   // cells (k*pitch + j) still iterating
+  uint32_t* cells;  // the mask's solve cells (k*pitch + j) on grids of DENSE_MIN_GRID cells, else null
   // learned warm start (warm != 0): the Newton cells of the step, their
   // network inputs and the network's momentum guesses
   int warm;
@@ -2267,14 +2293,28 @@ struct NewtonShared {
   NewtonStats st;
 };
 
-// Steps with at least this many solve cells leave some cells to the compacted
-// list of k_stage2_rest (LIST): those that the lean Jacobian does not cover
-// (the rest's code evicts the others', see k_stage2: 2.03+0.07 against 3.24 ms
-// on 2048^2 cells of the fractal workload, 0.55+0.05 against 0.75 on 1024^2,
-// equal on 512^2), and a warp's last few iterating lanes.  Below, the
-// list costs more than it saves (160 thousand solve cells of a 1024^2 grid:
-// 0.235+0.036 ms with it, 0.207 without; on a slope 0.28 and 0.09 ms).
+// Steps that solve at least this many cells, and half of the grid or more, leave
+// some cells to the compacted list of k_stage2_rest (LIST): those that the lean
+// Jacobian does not cover (the rest's code evicts the others', see k_stage2), and
+// a warp's last few iterating lanes.  The line lies between the states that gain
+// and those that lose (ms per step with the list / without): a layer of 600^2 cells
+// 0.487 / 0.462, 720^2 0.659 / 0.643, 900^2 0.979 / 0.978, 1024^2 1.230 / 1.251,
+// 2048^2 4.57 / 4.85; a layer on a slope after 60 steps, 700^2 0.589 / 0.600, 850^2
+// 0.797 / 0.852; a dam break of 2048^2 cells, most of them in one iteration, 2.01 /
+// 1.75.  Steps that solve less than half of the grid never take it: a radial
+// current of 1600^2 cells 0.733 / 0.530, a slope of 2048^2 1.33 / 1.12.
 constexpr unsigned long long LIST_MIN_CELLS = 1 << 18;
+// On grids of at least this many cells (more than the 512 threads per SM that
+// k_stage2 has in flight) the mask pass lists its solve cells, and a step
+// that solves less than half of the grid takes stage 2 over that list: blocks
+// of solve cells only, in place of grid rows that the current covers in part.
+// A block lasts as long as its slowest cell, up to ten iterations, so that
+// the number of blocks decides.  Stage 2 of the radial current of 1024^2 cells
+// after 1000 steps (84367 solve cells, 2952 of 8192 grid blocks touched): 0.277 ms
+// against 0.431 over the grid, after 300 steps (28143) 0.270 against 0.301; a
+// slope of 512^2 (45728) 0.116 against 0.132.  The list costs the mask pass
+// 0.003 ms on 1024^2 cells.
+constexpr unsigned long long DENSE_MIN_GRID = 148 * 512;
 // Lanes still iterating at or below which a warp leaves them to the list: going on
 // costs the whole warp an iteration, the list about sixty loads and stores per
 // cell (2: 2.05 ms, 6: 2.27 ms, 12: 2.29 ms in the first example above).
@@ -2384,6 +2424,24 @@ __device__ __forceinline__ void stage2_lane(
   }
 }
 
+// Whether stage 2 takes the mask's list: complete (a mask that was not
+// listed, or not to its end, has n_listed below solve_cells) and less than half of
+// the grid.
+__device__ __forceinline__ bool mask_is_sparse_list(const DevParams& P, const NewtonWork& W,
+                                                    const DevClock* clk) {
+  return W.cells && clk->n_listed == clk->solve_cells &&
+         2 * clk->solve_cells < (unsigned long long)P.nx * P.ny;
+}
+
+// Empties the list of remaining cells and chooses k_stage2's form for this step, on
+// grids that can reach LIST_MIN_CELLS (the same tests in k_stage2<.., true>
+// itself cost it 1%: 2.129 against 2.110 ms on 2048^2 cells).
+__global__ void k_stage2_form(const __grid_constant__ DevParams P,
+                              const __grid_constant__ NewtonWork W, DevClock* clk) {
+  clk->nw_count[0] = 0;
+  clk->use_list = !mask_is_sparse_list(P, W, clk) && clk->solve_cells >= LIST_MIN_CELLS;
+}
+
 // Stage 2 over the grid rows [k0, k1), of the steps whose number of solve cells
 // asks for LIST (the other kernel returns at once): blocks of T threads, 512
 // per SM, at 128 registers (84 registers spilled 2 kB per thread and measured 2.58
@@ -2409,21 +2467,33 @@ __global__ void __launch_bounds__(T, 512 / T)
              const double* __restrict__ By, const double* __restrict__ Bxx,
              const double* __restrict__ Bxy, const double* __restrict__ Byy,
              const double* __restrict__ gc, const __grid_constant__ NewtonWork W, DevClock* clk,
-             int k0, int k1, unsigned long long list_min) {
+             int k0, int k1, bool list_form) {
   const DevParams& P = Pp;
-  if ((clk->solve_cells >= list_min) != LIST) return;
+  if (list_form && (clk->use_list != 0) != LIST) return;
+  const bool dense = !LIST && mask_is_sparse_list(P, W, clk);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   NewtonShared<NS, T>& S = *reinterpret_cast<NewtonShared<NS, T>*>(smem_raw);
   const int nx = P.nx;
   const long long ncell = (long long)nx * (k1 - k0);
+  const long long n = dense ? (long long)clk->solve_cells : ncell;
+  if ((long long)blockIdx.x * blockDim.x >= n) return;
   const double dt = clk->dt;
   stat_reset(S.st, threadIdx.x);
   __syncthreads();
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x; base < ncell; base += stride) {
+  for (long long base = (long long)blockIdx.x * blockDim.x; base < n; base += stride) {
     const long long g = base + threadIdx.x;
+    int j, k;
+    if (dense) {
+      const uint32_t c = g < n ? W.cells[g] : 0;
+      j = (int)(c % (unsigned)P.pitch);
+      k = (int)(c / (unsigned)P.pitch);
+    } else {
+      j = (int)(g % nx);
+      k = k0 + (int)(g / nx);
+    }
     stage2_lane<NS, T, LIST>(P, S, q, X, mask, cellinfo, Bx, By, Bxx, Bxy, Byy, gc, W, clk, dt,
-                             g < ncell, (int)(g % nx), k0 + (int)(g / nx));
+                             g < n, j, k);
   }
   __syncthreads();
   stat_flush(S.st, clk, threadIdx.x);
@@ -2929,10 +2999,18 @@ __global__ void k_fp64_probe(double* out, int iters, double a, double b) {
   if (r == 12345.678) out[0] = r;  // keeps the chains live
 }
 
-// Resets the per-step accumulators of the clock.
-__device__ __forceinline__ void step_begin(DevClock* clk, double max_dt, int reset_cells) {
+// Resets the per-step accumulators of the clock.  The mask pass lists its
+// solve cells (n_listed below half of the grid's ncell) unless the mask before
+// was listed and held half of the grid or more: a list that will not be used
+// costs it 0.012 of 0.065 ms on 2048^2 cells.  (A new state's all-cells mask is
+// not listed and says nothing of the next one.)
+__device__ __forceinline__ void step_begin(DevClock* clk, double max_dt, int reset_cells,
+                                           unsigned long long ncell) {
   clk->dtmin_bits = (unsigned long long)__double_as_longlong(max_dt);
-  if (reset_cells) clk->solve_cells = 0;
+  if (reset_cells) {
+    clk->n_listed = (clk->n_listed == 0 || 2 * clk->solve_cells < ncell) ? 0 : 1ULL << 62;
+    clk->solve_cells = 0;
+  }
   clk->newton_cells = 0;
   clk->newton_iters = 0;
   clk->lnsrch_trials = 0;
@@ -2941,8 +3019,9 @@ __device__ __forceinline__ void step_begin(DevClock* clk, double max_dt, int res
   for (int b = 0; b < 16; ++b) clk->hist[b] = 0;
 }
 
-__global__ void k_step_begin(DevClock* clk, double max_dt, int reset_cells) {
-  step_begin(clk, max_dt, reset_cells);
+__global__ void k_step_begin(DevClock* clk, double max_dt, int reset_cells,
+                             unsigned long long ncell) {
+  step_begin(clk, max_dt, reset_cells, ncell);
 }
 
 // Empties the stage-2 Newton lists (before each stage 2).

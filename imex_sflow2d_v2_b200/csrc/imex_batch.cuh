@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
     }
     const long long e = (long long)(base - off[m]) + lane;
     stage2_rest_lane<NS>(wP, D.q, D.cellinfo, D.Bx, D.By, D.W, D.clk, D.clk->dt,
-                         e < (long long)D.clk->nw_count[0], e, true, st);
+                         e < (long long)D.clk->nw_count[0], e, st);
   }
   __syncwarp();
   if (cur >= 0) stat_flush(st, M[cur].clk, lane);

@@ -161,7 +161,7 @@ int grid_1d(long long n, int threads) {
 enum {
   KID_MASK = 0,
   KID_FLUX = 1,
-  KID_S2_FIRST = 2,   // stage 2 (with the learned start or harvest: up to iteration 1)
+  KID_S2_FIRST = 2,   // stage 2 (with the learned start or harvest: up to the solve)
   KID_S2_ITER = 3,    // the Newton iterations left to the list
   KID_S2_POST = 4,    // sign guard and assembly (learned start, harvest)
   KID_EROSION = 5,
@@ -318,7 +318,7 @@ cudaError_t launch_stage2_rows(ImexCtx* ctx, int k0, int k1) {
   // one resident wave over the list
   const int grid = grid_1d((long long)P.nx * (k1 - k0), STAGE2_THREADS);
   k_stage2_rest<NS><<<std::min(grid, 148 * IMEX_REST_MINB), STAGE2_THREADS, 0, ctx->stream>>>(
-      ctx->P, ctx->q, ctx->cellinfo, ctx->Bx, ctx->By, ctx->nw, ctx->clk, 1);
+      ctx->P, ctx->q, ctx->cellinfo, ctx->Bx, ctx->By, ctx->nw, ctx->clk);
   ctx->launches += 1;
   return cudaGetLastError();
 }
@@ -329,8 +329,6 @@ cudaError_t launch_stage2_ns(ImexCtx* ctx) {
   if (!ctx->nw.warm && !ctx->nw.harvest) return launch_stage2_rows<NS>(ctx, 0, P.ny);
   const long long ncell = (long long)P.nx * P.ny;
   const int grid = grid_1d(ncell, STAGE2_THREADS);
-  // list passes: one resident wave, grid-stride
-  const int lgrid = std::min(grid, 148 * IMEX_REST_MINB);
   k_nw_reset<<<1, 1, 0, ctx->stream>>>(ctx->clk);
   {
     ProfScope ps(ctx, KID_S2_FIRST);
@@ -340,18 +338,17 @@ cudaError_t launch_stage2_ns(ImexCtx* ctx) {
     if (ctx->nw.warm) {
       cudaError_t e = launch_warm_predict(ctx);
       if (e != cudaSuccess) return e;
-      k_stage2_wstart<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx,
-                                                                     ctx->By, ctx->nw, ctx->clk);
-      ctx->launches += 1;
     }
   }
   {
     ProfScope ps(ctx, KID_S2_ITER);
-    k_stage2_rest<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(
-        ctx->P, ctx->q, ctx->cellinfo, ctx->Bx, ctx->By, ctx->nw, ctx->clk, 0);
+    // the number of cells is known on the device only: blocks past it return at once
+    k_stage2_solve<NS><<<grid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx, ctx->By,
+                                                                 ctx->nw, ctx->clk);
     if (ctx->nw.warm) {
-      k_stage2_fallback<NS><<<lgrid, STAGE2_THREADS, 0, ctx->stream>>>(ctx->P, ctx->q, ctx->Bx,
-                                                                       ctx->By, ctx->nw, ctx->clk);
+      // one resident wave over the list
+      k_stage2_fallback<NS><<<std::min(grid, 148 * IMEX_REST_MINB), STAGE2_THREADS, 0,
+                              ctx->stream>>>(ctx->P, ctx->q, ctx->Bx, ctx->By, ctx->nw, ctx->clk);
       ctx->launches += 1;
     }
   }

@@ -1967,10 +1967,9 @@ __device__ bool erosion_cell(const DevParams& P, double* qc, double bx, double b
 //                    written: one thread per cell, its vectors in shared memory
 //   k_stage2_rest    on large grids, the cells that k_stage2 left iterating
 //                    when few lanes of their warp were, compacted in a list
-// With the learned start or its harvest the solve is cut where those need it:
-// k_stage2_first (up to iteration 1, or to the network's inputs), the network and
-// k_stage2_wstart, k_stage2_rest over the list of the cells still iterating,
-// k_stage2_post (sign guard and assembly).
+// With the learned start or its harvest stage 2 is cut where those need it:
+// k_stage2_first (up to the solve), the network, k_stage2_solve, k_stage2_post (sign guard
+// and assembly).
 // Between kernels a cell's Newton state (qj_rel, the residual, its norm) is
 // kept in the NewtonWork planes; the iterate is carried bit for bit, so a
 // cell's arithmetic is that of one uninterrupted solve_rk_step.
@@ -2500,24 +2499,20 @@ __global__ void __launch_bounds__(T, 512 / T)
 }
 
 // The remaining iterations of entry e of the list (valid: e is inside the
-// list).  `assemble`: sign guard and assembly follow here (k_stage2's cells), else
-// the result goes to W.x.
+// list), the sign guard and the assembly.
 template <int NS>
 __device__ __forceinline__ void stage2_rest_lane(const DevParams& P, double* __restrict__ q,
                                                  const uint8_t* __restrict__ cellinfo,
                                                  const double* __restrict__ Bx,
                                                  const double* __restrict__ By,
                                                  const NewtonWork& W, DevClock* clk, double dt,
-                                                 bool valid, long long e, bool assemble,
-                                                 NewtonStats& st) {
+                                                 bool valid, long long e, NewtonStats& st) {
   constexpr int NV = 4 + NS;
   const size_t N = (size_t)P.plane;
   int fin = 0;
-  bool fb = false;
-  uint32_t c = 0;
   unsigned tr = 0;
   if (valid) {
-    c = W.list[e];
+    const uint32_t c = W.list[e];
     double q0[NV], Rj[NV], qj_org[NV], qj_rel[NV], rt[NV], qj[NV], scal_f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -2528,10 +2523,6 @@ __device__ __forceinline__ void stage2_rest_lane(const DevParams& P, double* __r
       rt[i] = W.rt[c + i * N];
     }
     const double qs1 = qj[1], qs2 = qj[2];
-    if (W.warm) {   // the Newton start (scaling source) was the network's guess
-      qj[1] = W.guess[c];
-      qj[2] = W.guess[c + N];
-    }
     scal_f = W.sf[c];
     const int status = W.status[c];
     bool stale = (status & 2) != 0, done;
@@ -2540,20 +2531,10 @@ __device__ __forceinline__ void stage2_rest_lane(const DevParams& P, double* __r
                                rt, scal_f, tr, stale, done);
 #pragma unroll
     for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
-    if (assemble) {
-      stage2_assemble<NS>(P, qj, true, qs1, qs2, q, cellinfo, clk, (int)(c % P.pitch),
-                          (int)(c / P.pitch));
-    } else {
-      fb = W.warm && (!done || !all_finite<NS>(qj));
-      W.status[c] = 1;
-      if (!fb) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) W.x[c + i * N] = qj[i];
-      }
-    }
+    stage2_assemble<NS>(P, qj, true, qs1, qs2, q, cellinfo, clk, (int)(c % P.pitch),
+                        (int)(c / P.pitch));
   }
   stat_add(st, false, fin, tr);
-  if (W.warm) list_append(fb, c, W.flist, &clk->nw_fb);
 }
 
 #ifndef IMEX_REST_MINB
@@ -2564,7 +2545,7 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
     k_stage2_rest(const __grid_constant__ DevParams Pp, double* __restrict__ q,
                   const uint8_t* __restrict__ cellinfo, const double* __restrict__ Bx,
                   const double* __restrict__ By, const __grid_constant__ NewtonWork W,
-                  DevClock* clk, int assemble) {
+                  DevClock* clk) {
   __shared__ NewtonStats st;
   const long long n = (long long)clk->nw_count[0];
   if ((long long)blockIdx.x * blockDim.x >= n) return;
@@ -2575,17 +2556,17 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
   for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n;
        base += stride) {
     const long long e = base + (threadIdx.x & 31);
-    stage2_rest_lane<NS>(Pp, q, cellinfo, Bx, By, W, clk, dt, e < n, e, assemble != 0, st);
+    stage2_rest_lane<NS>(Pp, q, cellinfo, Bx, By, W, clk, dt, e < n, e, st);
   }
   __syncthreads();
   stat_flush(st, clk, threadIdx.x);
 }
 
-// Stage 2 up to Newton iteration 1, or with the learned start up to the
-// network's inputs, keeping q_si, Rj and the Newton state in the NewtonWork
-// planes.
+// Stage 2 up to the Newton solve, for the learned start and the harvest: q_si and Rj to
+// the NewtonWork planes, the cells to solve to a list (with the learned start the
+// one that also holds the network's inputs).
 #ifndef IMEX_FIRST_MINB
-#define IMEX_FIRST_MINB 5
+#define IMEX_FIRST_MINB 6
 #endif
 template <int NS>
 __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_FIRST_MINB)
@@ -2610,9 +2591,7 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_FIRST_MINB)
     const long long g = base + (threadIdx.x & 31);
     const bool valid = g < ncell;
     const size_t c = valid ? (size_t)(g / nx) * P.pitch + (size_t)(g % nx) : 0;
-    bool newton = false, go_on = false, warm_cell = false;
-    int fin = 0;
-    unsigned tr = 0;
+    bool newton = false;
     float fw[WARM_IN];
     if (valid && mask[c]) {
       double q0[NV], Xc[NV], qsi[NV], Rj[NV], bx, by;
@@ -2630,45 +2609,21 @@ __global__ void __launch_bounds__(STAGE2_THREADS, IMEX_FIRST_MINB)
           W.Rj[c + i * N] = Rj[i];
         }
       }
-      if (newton && W.warm) {
-        // Newton waits for the network's guess (k_warm_predict, k_stage2_wstart)
-        warm_features<NS>(qsi, q0, Rj, dt, bx, by, fw);
-        warm_cell = true;
-      } else {
-        if (newton) {
-          double qj_org[NV], qj_rel[NV], rt[NV], scal_f;
-          bool need_rt, stale = false;
-          if (newton_begin<NS, 1>(P, qsi, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f, need_rt) ||
-              newton_step<NS, 1>(P, true, need_rt, q0, Rj, qj_org, bx, by, dt, qj_rel, rt, scal_f,
-                                 tr, stale)) {
-            fin = 1;
+      if (newton && W.warm) warm_features<NS>(qsi, q0, Rj, dt, bx, by, fw);
+      if (!newton) {
 #pragma unroll
-            for (int i = 0; i < NV; ++i) qsi[i] = qj_rel[i] * qj_org[i];
-          } else {
-            go_on = true;
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-              W.x[c + i * N] = qj_rel[i];
-              W.rt[c + i * N] = rt[i];
-            }
-            W.sf[c] = scal_f;
-            W.status[c] = (1 << 2) | 1;
-          }
-        }
-        if (!go_on) {
-#pragma unroll
-          for (int i = 0; i < NV; ++i) W.x[c + i * N] = qsi[i];
-        }
+        for (int i = 0; i < NV; ++i) W.x[c + i * N] = qsi[i];
       }
     }
-    stat_add(st, newton, fin, tr);
-    list_append(go_on, (uint32_t)c, W.list, &clk->nw_count[0]);
+    stat_add(st, newton, 0, 0);
     if (W.warm) {
-      const unsigned int slot = list_append(warm_cell, (uint32_t)c, W.wlist, &clk->nw_count[3]);
-      if (warm_cell) {
+      const unsigned int slot = list_append(newton, (uint32_t)c, W.wlist, &clk->nw_count[3]);
+      if (newton) {
 #pragma unroll
         for (int i = 0; i < WARM_IN; ++i) W.feat[(size_t)slot * WARM_IN + i] = fw[i];
       }
+    } else {
+      list_append(newton, (uint32_t)c, W.list, &clk->nw_count[0]);
     }
   }
   __syncthreads();
@@ -2717,74 +2672,78 @@ __global__ void __launch_bounds__(32 * mlp::WARPS)
   }
 }
 
-// Newton scaling and iteration 1 from the network's guess for the cells of
-// the warm-start list; cells still iterating go to the list as in
-// k_stage2_first.
+// The Newton solves of k_stage2_first's list, from the network's guess or from q_si:
+// the iterations of stage2_lane, the block's warps together; results to
+// W.x, failed warm starts to the fallback list.  Bound as k_stage2 is; it takes the
+// place of iteration 1 in the kernel before and the others lane by lane
+// over a list: 0.157 + 0.268 ms on 163 thousand cells of a 1024^2 radial current,
+// 0.031 + 0.310 now, 0.261 + 0.392 on a layer of 1024^2 cells, 0.072 + 0.502 now.
 template <int NS>
-__global__ void __launch_bounds__(STAGE2_THREADS, IMEX_REST_MINB)
-    k_stage2_wstart(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
-                    const double* __restrict__ Bx, const double* __restrict__ By,
-                    const __grid_constant__ NewtonWork W, DevClock* clk) {
+__global__ void __launch_bounds__(STAGE2_THREADS, 512 / STAGE2_THREADS)
+    k_stage2_solve(const __grid_constant__ DevParams Pp, const double* __restrict__ q,
+                   const double* __restrict__ Bx, const double* __restrict__ By,
+                   const __grid_constant__ NewtonWork W, DevClock* clk) {
   const DevParams& P = Pp;
-  constexpr int NV = 4 + NS;
-  __shared__ NewtonStats st;
+  constexpr int NV = 4 + NS, ST = STAGE2_THREADS;
+  __shared__ NewtonShared<NS, ST> S;
+  const long long n = (long long)clk->nw_count[W.warm ? 3 : 0];
+  if ((long long)blockIdx.x * ST >= n) return;
+  const uint32_t* cells = W.warm ? W.wlist : W.list;
   const size_t N = (size_t)P.plane;
   const double dt = clk->dt;
-  const long long n = (long long)clk->nw_count[3];
-  stat_reset(st, threadIdx.x);
+  double* q0 = &S.q0[0][threadIdx.x];
+  double* Rj = &S.Rj[0][threadIdx.x];
+  double* org = &S.org[0][threadIdx.x];
+  stat_reset(S.st, threadIdx.x);
   __syncthreads();
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n;
-       base += stride) {
-    const long long e = base + (threadIdx.x & 31);
-    uint32_t c = 0;
-    bool go_on = false, fb = false;
-    int fin = 0;
-    unsigned tr = 0;
-    if (e < n) {
-      c = W.wlist[e];
-      double q0[NV], Rj[NV], qj[NV], qj_org[NV], qj_rel[NV], rt[NV], scal_f;
+  for (long long base = (long long)blockIdx.x * ST; base < n; base += (long long)gridDim.x * ST) {
+    const bool valid = base + threadIdx.x < n;
+    const uint32_t c = valid ? cells[base + threadIdx.x] : 0;
+    double rel[NV], rt[NV], scal_f = 0.0, bx = 0.0, by = 0.0;
+    bool go = false, need_rt = false, stale = false, fb = false;
+    int it = 0;
+    unsigned trials = 0;
+    if (valid) {
+      double g[NV];
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        q0[i] = q[c + i * N];
-        Rj[i] = W.Rj[c + i * N];
-        qj[i] = W.qsi[c + i * N];
+        q0[i * ST] = q[c + i * N];
+        Rj[i * ST] = W.Rj[c + i * N];
+        g[i] = W.qsi[c + i * N];
       }
-      qj[1] = W.guess[c];
-      qj[2] = W.guess[c + N];
-      const double bx = Bx[c], by = By[c];
-      bool need_rt, stale = false;
-      const bool done =
-          newton_begin<NS, 1>(P, qj, q0, Rj, bx, by, dt, qj_org, qj_rel, rt, scal_f, need_rt) ||
-          newton_step<NS, 1>(P, true, need_rt, q0, Rj, qj_org, bx, by, dt, qj_rel, rt, scal_f, tr,
-                             stale);
-      if (done) {
-        fin = 1;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) qj[i] = qj_rel[i] * qj_org[i];
-        if (!all_finite<NS>(qj)) {
-          fb = true;
-        } else {
-#pragma unroll
-          for (int i = 0; i < NV; ++i) W.x[c + i * N] = qj[i];
-        }
-      } else {
-        go_on = true;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          W.x[c + i * N] = qj_rel[i];
-          W.rt[c + i * N] = rt[i];
-        }
-        W.sf[c] = scal_f;
-        W.status[c] = (1 << 2) | 1;
+      if (W.warm) {
+        g[1] = W.guess[c];
+        g[2] = W.guess[c + N];
+      }
+      bx = Bx[c];
+      by = By[c];
+      go = !newton_begin<NS, ST>(P, g, q0, Rj, bx, by, dt, org, rel, rt, scal_f, need_rt);
+    }
+#pragma unroll 1
+    for (int m = 1; m <= NEWTON_MAX_IT; ++m) {
+      if (!__syncthreads_or(go)) break;
+      if (go) {
+        go = !newton_step<NS, ST>(P, m == 1, need_rt, q0, Rj, org, bx, by, dt, rel, rt, scal_f,
+                                  trials, stale);
+        need_rt = false;
+        it = m;
       }
     }
-    stat_add(st, false, fin, tr);
-    list_append(go_on, c, W.list, &clk->nw_count[0]);
-    list_append(fb, c, W.flist, &clk->nw_fb);
+    if (valid) {
+      double qj[NV];
+#pragma unroll
+      for (int i = 0; i < NV; ++i) qj[i] = rel[i] * org[i * ST];
+      fb = W.warm && (go || !all_finite<NS>(qj));   // go: not converged in 100 iterations
+      if (!fb) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) W.x[c + i * N] = qj[i];
+      }
+    }
+    stat_add(S.st, false, valid ? max(it, 1) : 0, trials);
+    if (W.warm) list_append(fb, c, W.flist, &clk->nw_fb);
   }
   __syncthreads();
-  stat_flush(st, clk, threadIdx.x);
+  stat_flush(S.st, clk, threadIdx.x);
 }
 
 // Warm starts that failed, redone with the plain start (q_si).

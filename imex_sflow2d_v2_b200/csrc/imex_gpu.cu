@@ -1518,8 +1518,23 @@ namespace {
 
 int mlp_fail(ImexMLP* m, int code, const std::string& msg) {
   if (m) m->last_error = msg;
+  cudaGetLastError();   // reported here, not by the next call's launch check
   return code;
 }
+// Device memory of one call, given back on every return.
+struct CallBuffer {
+  void* p = nullptr;
+  ~CallBuffer() {
+    if (p) cudaFree(p);
+  }
+  template <class T>
+  cudaError_t alloc(T** out, size_t n) {
+    const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+    *out = static_cast<T*>(p);
+    return e;
+  }
+};
+
 #define CKM(call)                                                             \
   do {                                                                        \
     cudaError_t e_ = (call);                                                  \
@@ -1641,9 +1656,10 @@ int imex_mlp_predict(ImexMLP* mlp, const float* x, int64_t n, float* y) {
   if (!mlp || !x || !y || n < 0) return IMEX_EINVAL;
   if (n == 0) return IMEX_OK;
   CKM(cudaSetDevice(mlp->device));
+  CallBuffer bx, by;
   float *dx = nullptr, *dy = nullptr;
-  CKM(cudaMalloc((void**)&dx, n * mlp::IN * sizeof(float)));
-  CKM(cudaMalloc((void**)&dy, n * mlp::OUT * sizeof(float)));
+  CKM(bx.alloc(&dx, (size_t)n * mlp::IN));
+  CKM(by.alloc(&dy, (size_t)n * mlp::OUT));
   CKM(cudaMemcpy(dx, x, n * mlp::IN * sizeof(float), cudaMemcpyHostToDevice));
   CKM(cudaFuncSetAttribute(mlp::k_mlp_predict, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)mlp::SMEM_NET));
@@ -1652,8 +1668,6 @@ int imex_mlp_predict(ImexMLP* mlp, const float* x, int64_t n, float* y) {
       mlp->bw, mlp->prm, dx, dy, n);
   CKM(cudaGetLastError());
   CKM(cudaMemcpy(y, dy, n * mlp::OUT * sizeof(float), cudaMemcpyDeviceToHost));
-  cudaFree(dx);
-  cudaFree(dy);
   return IMEX_OK;
 }
 
@@ -1661,9 +1675,10 @@ int imex_mlp_loss_grad(ImexMLP* mlp, const float* x, const float* y, int64_t n, 
                        float* grad) {
   if (!mlp || !x || !y || n <= 0) return IMEX_EINVAL;
   CKM(cudaSetDevice(mlp->device));
+  CallBuffer bx, by;
   float *dx = nullptr, *dy = nullptr;
-  CKM(cudaMalloc((void**)&dx, n * mlp::IN * sizeof(float)));
-  CKM(cudaMalloc((void**)&dy, n * mlp::OUT * sizeof(float)));
+  CKM(bx.alloc(&dx, (size_t)n * mlp::IN));
+  CKM(by.alloc(&dy, (size_t)n * mlp::OUT));
   CKM(cudaMemcpy(dx, x, n * mlp::IN * sizeof(float), cudaMemcpyHostToDevice));
   CKM(cudaMemcpy(dy, y, n * mlp::OUT * sizeof(float), cudaMemcpyHostToDevice));
   CKM(cudaMemset(mlp->grad, 0, mlp::NPARAM * sizeof(float)));
@@ -1674,8 +1689,6 @@ int imex_mlp_loss_grad(ImexMLP* mlp, const float* x, const float* y, int64_t n, 
   if (loss) *loss = ls / (float)(n * mlp::OUT);
   if (grad) CKM(cudaMemcpy(grad, mlp->grad, mlp::NPARAM * sizeof(float), cudaMemcpyDeviceToHost));
   CKM(cudaMemset(mlp->grad, 0, mlp::NPARAM * sizeof(float)));
-  cudaFree(dx);
-  cudaFree(dy);
   return IMEX_OK;
 }
 
@@ -1692,11 +1705,12 @@ int imex_mlp_train(ImexMLP* mlp, const float* x_dev, const float* y_dev, int64_t
     long long j = (long long)(splitmix64(st) % (uint64_t)(i + 1));
     std::swap(perm[i], perm[j]);
   }
+  CallBuffer bp, bx, by;
   long long* dperm = nullptr;
   float *xs = nullptr, *ys = nullptr;
-  CKM(cudaMalloc((void**)&dperm, n * sizeof(long long)));
-  CKM(cudaMalloc((void**)&xs, n * mlp::IN * sizeof(float)));
-  CKM(cudaMalloc((void**)&ys, n * mlp::OUT * sizeof(float)));
+  CKM(bp.alloc(&dperm, (size_t)n));
+  CKM(bx.alloc(&xs, (size_t)n * mlp::IN));
+  CKM(by.alloc(&ys, (size_t)n * mlp::OUT));
   CKM(cudaMemcpy(dperm, perm.data(), n * sizeof(long long), cudaMemcpyHostToDevice));
   mlp::k_gather_rows<<<148 * 8, 256>>>(x_dev, dperm, xs, n, mlp::IN);
   mlp::k_gather_rows<<<148 * 8, 256>>>(y_dev, dperm, ys, n, mlp::OUT);
@@ -1722,9 +1736,6 @@ int imex_mlp_train(ImexMLP* mlp, const float* x_dev, const float* y_dev, int64_t
     if (loss_out) loss_out[e] = (float)(esum / (double)(n * mlp::OUT));
   }
   CKM(cudaDeviceSynchronize());
-  cudaFree(dperm);
-  cudaFree(xs);
-  cudaFree(ys);
   return IMEX_OK;
 }
 

@@ -76,7 +76,7 @@ __global__ void kb_step_begin(MemberDev* M, int n, unsigned int* n_active) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m == 0) *n_active = 0;
   if (m < n) {
-    step_begin(M[m].clk, M[m].P.max_dt, 1, (unsigned long long)M[m].P.nx * M[m].P.ny);
+    step_begin(M[m].clk, M[m].P.max_dt, 1, 0);
     nw_reset(M[m].clk);
   }
 }

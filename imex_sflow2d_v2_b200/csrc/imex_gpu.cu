@@ -150,6 +150,11 @@ cudaError_t upload_plane(ImexCtx* ctx, double* dst, const double* src, double fi
 
 unsigned long long grid_cells(const DevParams& P) { return (unsigned long long)P.nx * P.ny; }
 
+// The grid's cells if stage 2 has two forms to choose from, else 0.
+unsigned long long form_cells(const DevParams& P) {
+  return grid_cells(P) >= LIST_MIN_CELLS ? grid_cells(P) : 0;
+}
+
 dim3 tile_grid(const DevParams& P) { return dim3((P.nx + TX - 1) / TX, (P.ny + TY - 1) / TY); }
 
 int grid_1d(long long n, int threads) {
@@ -301,11 +306,11 @@ template <int NS>
 cudaError_t launch_stage2_rows(ImexCtx* ctx, int k0, int k1) {
   const DevParams& P = ctx->P;
   cudaError_t e;
-  if ((long long)P.nx * P.ny < (long long)LIST_MIN_CELLS) {
+  if (!form_cells(P)) {
     ProfScope ps(ctx, KID_S2_FIRST);
     return launch_stage2_blocks<NS, STAGE2_THREADS, false>(ctx, k0, k1, false);
   }
-  k_stage2_form<<<1, 1, 0, ctx->stream>>>(ctx->P, ctx->nw, ctx->clk);
+  k_nw_reset<<<1, 1, 0, ctx->stream>>>(ctx->clk);
   ctx->launches += 1;
   {
     ProfScope ps(ctx, KID_S2_FIRST);
@@ -458,7 +463,8 @@ bool erosion_active(const ImexCtx* ctx) {
 // , erosion/deposition, t += dt.
 cudaError_t enqueue_step(ImexCtx* ctx) {
   cudaError_t e;
-  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 1, grid_cells(ctx->P));
+  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 1,
+                                         ctx->nw.cells ? grid_cells(ctx->P) : 0);
   ctx->launches += 1;
   {
     ProfScope ps(ctx, KID_MASK);
@@ -468,7 +474,7 @@ cudaError_t enqueue_step(ImexCtx* ctx) {
     ProfScope ps(ctx, KID_FLUX);
     if ((e = launch_flux(ctx)) != cudaSuccess) return e;
   }
-  k_dt_clip<<<1, 1, 0, ctx->stream>>>(ctx->clk, 1);
+  k_dt_clip<<<1, 1, 0, ctx->stream>>>(ctx->clk, 1, ctx->nw.cells, form_cells(ctx->P));
   ctx->launches += 1;
   if ((e = launch_stage2(ctx)) != cudaSuccess) return e;
   if (erosion_active(ctx)) {
@@ -523,7 +529,7 @@ cudaError_t enqueue_host_step_ns(ImexCtx* ctx, const double* q_in, double* q_out
       return e;
     if ((e = cudaEventRecord(ev[1 + b], cs)) != cudaSuccess) return e;
   }
-  k_step_begin<<<1, 1, 0, st>>>(ctx->clk, P.max_dt, 1, grid_cells(P));
+  k_step_begin<<<1, 1, 0, st>>>(ctx->clk, P.max_dt, 1, 0);
   const size_t smem = sizeof(FluxShared<NS>);
   static std::atomic<unsigned long long> attr_set{0};
   if (attr_needed(attr_set)) {
@@ -569,7 +575,7 @@ cudaError_t enqueue_host_step_ns(ImexCtx* ctx, const double* q_in, double* q_out
   mask_band(nb - 1);
   if (nb >= 2) flux_band(nb - 2);
   flux_band(nb - 1);
-  k_dt_clip<<<1, 1, 0, st>>>(ctx->clk, 1);
+  k_dt_clip<<<1, 1, 0, st>>>(ctx->clk, 1, ctx->nw.cells, form_cells(P));
   ++launches;
   const bool ero = erosion_active(ctx);
   for (int b = 0; b < nb; ++b) {
@@ -1092,13 +1098,13 @@ int imex_gpu_check_solve(ImexCtx* ctx, double t, int solve_all, int64_t* n_solve
 int imex_gpu_timestep(ImexCtx* ctx, double* dt) {
   if (!ctx || !dt) return IMEX_EINVAL;
   CK(cudaSetDevice(ctx->device));
-  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 0, grid_cells(ctx->P));
+  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->clk, ctx->P.max_dt, 0, 0);
   ctx->launches += 1;
   if (ctx->P.cfl != -1.0) {
     CK(launch_flux(ctx));
     ctx->x_valid = true;
   }
-  k_dt_clip<<<1, 1, 0, ctx->stream>>>(ctx->clk, 0);
+  k_dt_clip<<<1, 1, 0, ctx->stream>>>(ctx->clk, 0, nullptr, 0);
   ctx->launches += 1;
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(dt, &ctx->clk->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1124,6 +1130,10 @@ int imex_gpu_rk_step(ImexCtx* ctx, double t, double dt) {
   int r = push_time(ctx, t, &dt);
   if (r) return r;
   if (!ctx->x_valid) CK(launch_flux(ctx));
+  if (form_cells(ctx->P)) {
+    k_stage2_form<<<1, 1, 0, ctx->stream>>>(ctx->nw.cells, grid_cells(ctx->P), ctx->clk);
+    ctx->launches += 1;
+  }
   CK(launch_stage2(ctx));
   ctx->x_valid = false;
   return collect_errors(ctx);

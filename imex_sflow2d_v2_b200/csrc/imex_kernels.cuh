@@ -78,7 +78,7 @@ struct DevClock {
   unsigned long long harvest_n;      // training pairs written so far
   unsigned long long warm_fallback;  // warm starts redone from q_si
   unsigned int nw_fb;                // cells in the warm-start fallback list
-  int use_list;                      // k_stage2's form in this step (k_stage2_form)
+  int use_list;                      // k_stage2's form (stage2_form)
 };
 
 IMEX_HD double x_stag(const DevParams& P, int J) { return P.x0 + (double)(J - 1) * P.dx; }
@@ -155,7 +155,6 @@ __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __re
   }
   __syncthreads();
   int cnt = 0;
-  size_t cell = 0;
   for (int e = threadIdx.x; e < TXt * TYt; e += blockDim.x) {
     int lx = e % TXt + HALO, ly = e / TXt + HALO;
     int j = j0 + lx - HALO, k = k0 + ly - HALO;
@@ -164,8 +163,7 @@ __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __re
     if (j >= 1 && j < nx - 1 && k >= 1 && k < ny - 1)
       m = m | s1[ly][lx - 1] | s1[ly][lx + 1] | s1[ly - 1][lx] | s1[ly + 1][lx];
     if (P.radial_source_flag && (cellinfo[(size_t)k * nx + j] & CI_SRC_MASK) == 1) m = 0;
-    cell = (size_t)k * P.pitch + j;
-    mask[cell] = m;
+    mask[(size_t)k * P.pitch + j] = m;
     cnt += m;
   }
   const bool solve = cnt != 0;
@@ -187,7 +185,8 @@ __device__ __forceinline__ bool mask_tile(const DevParams& P, const double* __re
     const unsigned m = __ballot_sync(0xffffffffu, solve);
     unsigned slot = first + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
     for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) slot += warp_cnt[w];
-    if (solve) cells[slot] = (uint32_t)cell;
+    if (solve)
+      cells[slot] = (uint32_t)((k0 + threadIdx.x / TXt) * P.pitch + j0 + threadIdx.x % TXt);
   }
   return total != 0;
 }
@@ -2426,19 +2425,20 @@ __device__ __forceinline__ void stage2_lane(
 // Whether stage 2 takes the mask's list: complete (a mask that was not
 // listed, or not to its end, has n_listed below solve_cells) and less than half of
 // the grid.
-__device__ __forceinline__ bool mask_is_sparse_list(const DevParams& P, const NewtonWork& W,
+__device__ __forceinline__ bool mask_is_sparse_list(const uint32_t* cells, unsigned long long ncell,
                                                     const DevClock* clk) {
-  return W.cells && clk->n_listed == clk->solve_cells &&
-         2 * clk->solve_cells < (unsigned long long)P.nx * P.ny;
+  return cells && clk->n_listed == clk->solve_cells && 2 * clk->solve_cells < ncell;
 }
 
-// Empties the list of remaining cells and chooses k_stage2's form for this step, on
-// grids that can reach LIST_MIN_CELLS (the same tests in k_stage2<.., true>
-// itself cost it 1%: 2.129 against 2.110 ms on 2048^2 cells).
-__global__ void k_stage2_form(const __grid_constant__ DevParams P,
-                              const __grid_constant__ NewtonWork W, DevClock* clk) {
-  clk->nw_count[0] = 0;
-  clk->use_list = !mask_is_sparse_list(P, W, clk) && clk->solve_cells >= LIST_MIN_CELLS;
+// k_stage2's form for the present mask (the same tests in k_stage2<.., true> itself
+// cost it 1%: 2.129 against 2.110 ms on 2048^2 cells).  A step takes them along in
+// k_dt_clip; either form solves any mask, so that a stale choice costs time only.
+__device__ __forceinline__ void stage2_form(const uint32_t* cells, unsigned long long ncell,
+                                            DevClock* clk) {
+  clk->use_list = !mask_is_sparse_list(cells, ncell, clk) && clk->solve_cells >= LIST_MIN_CELLS;
+}
+__global__ void k_stage2_form(const uint32_t* cells, unsigned long long ncell, DevClock* clk) {
+  stage2_form(cells, ncell, clk);
 }
 
 // Stage 2 over the grid rows [k0, k1), of the steps whose number of solve cells
@@ -2469,7 +2469,8 @@ __global__ void __launch_bounds__(T, 512 / T)
              int k0, int k1, bool list_form) {
   const DevParams& P = Pp;
   if (list_form && (clk->use_list != 0) != LIST) return;
-  const bool dense = !LIST && mask_is_sparse_list(P, W, clk);
+  const bool dense =
+      !LIST && mask_is_sparse_list(W.cells, (unsigned long long)P.nx * P.ny, clk);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   NewtonShared<NS, T>& S = *reinterpret_cast<NewtonShared<NS, T>*>(smem_raw);
   const int nx = P.nx;
@@ -2962,12 +2963,14 @@ __global__ void k_fp64_probe(double* out, int iters, double a, double b) {
 // solve cells (n_listed below half of the grid's ncell) unless the mask before
 // was listed and held half of the grid or more: a list that will not be used
 // costs it 0.012 of 0.065 ms on 2048^2 cells.  (A new state's all-cells mask is
-// not listed and says nothing of the next one.)
+// not listed and says nothing of the next one.)  ncell 0, where no mask is listed:
+// without the two loads, which one thread waits 0.6 us for.
 __device__ __forceinline__ void step_begin(DevClock* clk, double max_dt, int reset_cells,
                                            unsigned long long ncell) {
   clk->dtmin_bits = (unsigned long long)__double_as_longlong(max_dt);
   if (reset_cells) {
-    clk->n_listed = (clk->n_listed == 0 || 2 * clk->solve_cells < ncell) ? 0 : 1ULL << 62;
+    clk->n_listed =
+        (ncell == 0 || clk->n_listed == 0 || 2 * clk->solve_cells < ncell) ? 0 : 1ULL << 62;
     clk->solve_cells = 0;
   }
   clk->newton_cells = 0;
@@ -3003,7 +3006,11 @@ __device__ __forceinline__ void dt_clip(DevClock* clk, int clip) {
   }
   clk->dt = dt;
 }
-__global__ void k_dt_clip(DevClock* clk, int clip) { dt_clip(clk, clip); }
+// With ncell, on grids that can reach LIST_MIN_CELLS, also stage 2's form.
+__global__ void k_dt_clip(DevClock* clk, int clip, const uint32_t* cells, unsigned long long ncell) {
+  dt_clip(clk, clip);
+  if (ncell) stage2_form(cells, ncell, clk);
+}
 
 __device__ __forceinline__ void step_end(DevClock* clk) {
   clk->t = clk->t + clk->dt;

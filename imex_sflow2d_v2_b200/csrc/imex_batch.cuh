@@ -160,7 +160,10 @@ __global__ void __launch_bounds__(STAGE2_THREADS, 512 / STAGE2_THREADS)
   __shared__ DevParams sP;
   __shared__ NewtonShared<NS, STAGE2_THREADS> S;
   const unsigned int n = *n_active;
-  // the active tiles' cells bound the members' solve cells together
+  // the active tiles' cells bound the members' solve cells together.  The list pays in
+  // sparse members too (24 radial currents of 256^2 to 512^2, 10 steps: 14.7 ms
+  // with it, 16.6 without), and costs little in full ones (3 layers of 800^2 cells 1.82
+  // and 1.82 ms per step, 8 of 300^2 0.82 and 0.80).
   if (((unsigned long long)n * (unsigned)(tx * ty) >= LIST_MIN_CELLS) != LIST) return;
   const MemberDev* cur = nullptr;
   for (unsigned int a = blockIdx.x; a < n; a += gridDim.x) {

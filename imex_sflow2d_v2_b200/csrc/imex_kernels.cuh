@@ -2441,23 +2441,25 @@ __global__ void k_stage2_form(const uint32_t* cells, unsigned long long ncell, D
   stage2_form(cells, ncell, clk);
 }
 
-// Stage 2 over the grid rows [k0, k1), of the steps whose number of solve cells
-// asks for LIST (the other kernel returns at once): blocks of T threads, 512
+// Stage 2 over the grid rows [k0, k1), or over the mask's list of a sparse step; the
+// kernel of the other form returns at once.  Blocks of T threads, 512
 // per SM, at 128 registers (84 registers spilled 2 kB per thread and measured 2.58
 // against 2.04 ms on 2048^2 cells).
 // What bounds it is instruction fetch: the solve's code is larger than the
 // instruction cache, and warps at different places in it evict each other's
 // (1024^2 cells of the fractal workload, warps on their own: 54% hits, 7 of 15
-// stall cycles without an instruction).  So the warps of a block take each
+// stall cycles without an instruction; in step 94%).  So the warps of a block take each
 // phase together, and with LIST, where there is work for it, one block of 512
-// fills the SM: 2.03 ms on 2048^2 cells against 2.18 ms in blocks of 128,
-// which the smaller steps take (a 1024^2 grid with 15% wet cells 0.18 against
-// 0.23 ms).  Rolled Jacobian columns (2.14 ms), a state machine with one
-// place for residuals (2.34 ms) and 160 registers less spill (2.01 ms, but
-// 0.060 against 0.043 ms on 99x99) were no better.
+// fills the SM: 2.03 ms on 2048^2 cells against 2.18 ms in blocks of 128.  The other
+// steps take blocks of 128, which wait for fewer slow cells: against blocks of
+// 512, 0.271 to 0.296 ms on a radial current of 1024^2 cells after 300 steps (but
+// 0.282 to 0.274 after 1000), 0.116 to 0.123 on a slope of 512^2, 0.169 to 0.176 on a
+// layer of 512^2, 0.0170 to 0.0182 on a dam break of 200^2.  Rolled Jacobian
+// columns (2.14 ms), a state machine with one place for residuals (2.34 ms) and 160
+// registers less spill (2.01 ms, but 0.060 against 0.043 ms on 99x99) were no better.
 // The kernels that this replaces, one pass per Newton iteration over lists in
-// memory, took 3.55 ms on those 2048^2 cells, 0.281 ms on that 1024^2 grid (0.269
-// now) and 0.234 on a 301x517 slope (0.088).
+// memory, took 3.55 ms on those 2048^2 cells, 0.264 ms on that radial current after
+// 1000 steps and 0.234 on a 301x517 slope (0.088).
 template <int NS, int T, bool LIST>
 __global__ void __launch_bounds__(T, 512 / T)
     k_stage2(const __grid_constant__ DevParams Pp, double* __restrict__ q,

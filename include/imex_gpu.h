@@ -238,8 +238,8 @@ int imex_gpu_advance(ImexCtx* ctx, int n_steps, int use_graph, double* t);
  * overlapped with the step.  The grid goes up and comes back in row bands
  * on a second stream: the masks and fluxes of a band start as soon as the
  * band and its neighbour rows are on the device, and a band's rows return
- * once its assembly and erosion/deposition are done (stage 2's Newton
- * passes, which wait for the global dt, run on the whole grid in between).
+ * once its stage 2, which waits for the global dt, and its erosion/deposition
+ * are done.
  * q_in and q_out are q(n_vars, nx, ny) in Fortran order and may be the same
  * array; page-locked host memory lets the copies overlap.  Returns like
  * imex_gpu_advance (a reference check's code after the step completed).

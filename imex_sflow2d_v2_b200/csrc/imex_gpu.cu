@@ -105,7 +105,13 @@ namespace {
 
 int fail(ImexCtx* c, int code, const std::string& msg) {
   if (c) c->last_error = msg;
+  cudaGetLastError();   // reported here, not by the next call's launch check
   return code;
+}
+
+void drop_graph(ImexCtx* ctx) {
+  if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
+  if (ctx->graph) { cudaGraphDestroy(ctx->graph); ctx->graph = nullptr; }
 }
 
 #define CK(call)                                                              \
@@ -1414,10 +1420,12 @@ int imex_gpu_post_init(ImexCtx* ctx, int n_thickness_levels, const double* thick
   L.n_words = (nt * np + 31) / 32;
   CK(cudaSetDevice(ctx->device));
   const size_t plane = (size_t)ctx->P.plane;
-  if (!ctx->post_buf) {
-    CK(dalloc(&ctx->post_buf, plane * 4));
-    CK(dalloc(&ctx->post_diag, 4 + 4 * (size_t)DIAG_BLOCKS));
-  }
+  // off, here and in a captured step, until all buffers are there
+  CK(cudaStreamSynchronize(ctx->stream));
+  ctx->post_on = false;
+  drop_graph(ctx);
+  if (!ctx->post_diag) CK(dalloc(&ctx->post_diag, 4 + 4 * (size_t)DIAG_BLOCKS));
+  if (!ctx->post_buf) CK(dalloc(&ctx->post_buf, plane * 4));
   if (ctx->post_vuln) {
     cudaFree(ctx->post_vuln);
     ctx->post_vuln = nullptr;
@@ -1433,9 +1441,7 @@ int imex_gpu_post_init(ImexCtx* ctx, int n_thickness_levels, const double* thick
   if (ctx->post_vuln)
     CK(cudaMemsetAsync(ctx->post_vuln, 0, plane * L.n_words * sizeof(uint32_t), ctx->stream));
   CK(launch_post_sweep(ctx, 1));
-  // a captured step does not hold the sweep yet
-  if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
-  if (ctx->graph) { cudaGraphDestroy(ctx->graph); ctx->graph = nullptr; }
+  drop_graph(ctx);   // a captured step does not hold the sweep yet
   ctx->post_on = true;
   CK(cudaStreamSynchronize(ctx->stream));
   return IMEX_OK;
@@ -1791,11 +1797,6 @@ cudaError_t launch_warm_predict(ImexCtx* ctx) {
 }
 }  // namespace
 
-static void drop_graph(ImexCtx* ctx) {
-  if (ctx->graph_exec) { cudaGraphExecDestroy(ctx->graph_exec); ctx->graph_exec = nullptr; }
-  if (ctx->graph) { cudaGraphDestroy(ctx->graph); ctx->graph = nullptr; }
-}
-
 extern "C" {
 
 int imex_gpu_set_warmstart(ImexCtx* ctx, ImexMLP* net) {
@@ -1805,10 +1806,10 @@ int imex_gpu_set_warmstart(ImexCtx* ctx, ImexMLP* net) {
   if (net && net->device != ctx->device)
     return fail(ctx, IMEX_EINVAL, "imex_gpu_set_warmstart: network on another device");
   const size_t plane = (size_t)ctx->P.plane;
-  if (net && !ctx->nw_wlist) {
-    CK(dalloc(&ctx->nw_wlist, plane * 2));   // warm-start list, then fallback list
-    CK(dalloc(&ctx->nw_feat, plane * WARM_IN));
-    CK(dalloc(&ctx->nw_guess, plane * 2));
+  if (net) {
+    if (!ctx->nw_wlist) CK(dalloc(&ctx->nw_wlist, plane * 2));   // warm-start list, then fallback list
+    if (!ctx->nw_feat) CK(dalloc(&ctx->nw_feat, plane * WARM_IN));
+    if (!ctx->nw_guess) CK(dalloc(&ctx->nw_guess, plane * 2));
   }
   ctx->warm_mlp = net;
   ctx->nw.warm = net ? 1 : 0;
@@ -1821,9 +1822,15 @@ int imex_gpu_set_warmstart(ImexCtx* ctx, ImexMLP* net) {
 }
 
 int imex_gpu_harvest_start(ImexCtx* ctx, int64_t capacity, int stride) {
-  if (!ctx || capacity <= 0 || stride < 1) return IMEX_EINVAL;
+  if (!ctx || capacity <= 0 || capacity > INT64_MAX / 64 || stride < 1) return IMEX_EINVAL;
   CK(cudaSetDevice(ctx->device));
   CK(cudaStreamSynchronize(ctx->stream));
+  // off, here and in a captured step, until the new buffers are there
+  const unsigned long long zero = 0;
+  CK(cudaMemcpy(&ctx->clk->harvest_n, &zero, sizeof(zero), cudaMemcpyHostToDevice));
+  ctx->nw.harvest = 0;
+  ctx->nw.hcap = 0;
+  drop_graph(ctx);
   if (ctx->h_x) cudaFree(ctx->h_x);
   if (ctx->h_y) cudaFree(ctx->h_y);
   ctx->h_x = nullptr;
@@ -1835,9 +1842,6 @@ int imex_gpu_harvest_start(ImexCtx* ctx, int64_t capacity, int stride) {
   ctx->nw.hcap = (unsigned long long)capacity;
   ctx->nw.hx = ctx->h_x;
   ctx->nw.hy = ctx->h_y;
-  const unsigned long long zero = 0;
-  CK(cudaMemcpy(&ctx->clk->harvest_n, &zero, sizeof(zero), cudaMemcpyHostToDevice));
-  drop_graph(ctx);
   return IMEX_OK;
 }
 

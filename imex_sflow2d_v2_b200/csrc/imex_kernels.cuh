@@ -962,7 +962,8 @@ IMEX_FLAT bool interface_kt(const DevParams& P, const FluxShared<NS, TS>& S, int
     const double coef = quot(Rg, aP * aN, ok);
     // products rounded on their own in the contracted build too: a multiply-add
     // would round the two sides of the average differently, and the radial
-    // current amplifies that (relative L1 at step 500 2.2e-12 against 1.6e-12)
+    // current amplifies that (relative L1 at step 500, when this was written, 2.2e-12
+    // with multiply-adds and 1.6e-12 without; 1.0e-12 now)
     auto kt = [&](double fl, double fr, double cl, double cr) {
       return quot(Rg, __dmul_rn(aP, fl) - __dmul_rn(aN, fr), ok) + __dmul_rn(coef, cr - cl);
     };

@@ -108,7 +108,7 @@ def test_mask_of_a_banded_host_step_is_not_the_listed_one():
 
 def test_thinly_spread_cells_cost_like_packed_ones():
     """65536 wet cells of a 1024 x 1024 grid in stripes that touch every grid block, and in one square: the
-    stripes' solve cells (their margins included) are 2.4 times the square's."""
+    stripes' solve cells (their margins included) are twice the square's."""
     n = 1024
     stripes = np.broadcast_to((np.arange(n) % 64 < 4)[:, None], (n, n)).astype(float)
     square = np.zeros((n, n))
